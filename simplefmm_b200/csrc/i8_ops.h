@@ -40,6 +40,27 @@ SFMM_HD void real_nm(int r, int& n, int& m, int& im)
 // (leading byte offset), row groups 256 B apart (stride byte offset).
 SFMM_HD int canon_off(int row, int k) { return (row >> 3) * 256 + (k >> 4) * 128 + (row & 7) * 16 + (k & 15); }
 
+// Whether the two locals share one set of operator rows.  The field local's row
+// of a coefficient and the potential local's row of the same coefficient have
+// the same entries for source orders < p; the potential local adds order p.
+// (p + 2)^2 rows then serve both: all rows over the orders < p (first K steps),
+// the field local read, then order p alone (one K step of 2p + 1 values) added
+// for the potential local.  Below p = 7 the separate rows fit one 128-row chunk
+// and take no more K steps; from there on sharing saves them (128-row chunks x
+// K steps per slot, separate -> shared: p = 7 4 -> 3, 8 6 -> 3, 9 8 -> 4,
+// 10 12 -> 9, 11 15 -> 10, 12 18 -> 12).
+SFMM_HD bool i8_shared_rows(int p) { return p >= 7; }
+
+// Real column (real_nm index) at position pos of a moment row, -1 for padding.
+// Shared rows: the orders < p fill the first KB 32-byte steps, order p the next.
+SFMM_HD int i8_column(int pos, int p, int KB, bool shared)
+{
+    if (!shared) return pos < (p + 1) * (p + 1) ? pos : -1;
+    if (pos < 32 * KB) return pos < p * p ? pos : -1;
+    const int k = p * p + (pos - 32 * KB);
+    return k < (p + 1) * (p + 1) ? k : -1;
+}
+
 // Digit number scale of ND signed 8-bit digits: |x| <= 1 -> |round(x Q)| <= Q.
 template<int ND>
 struct I8Digits {

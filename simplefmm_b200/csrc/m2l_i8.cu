@@ -36,29 +36,45 @@
 // 216 slots in a 6 x 6 x 6 box.  A row block is up to 128 target rows
 // (target x charge component) of one group; its slot table lists each
 // target's source per slot.  The blocks of a level are numbered with the 8
-// octants of a region adjacent, so blocks that run together share sources.  A work item is a row block and 128 operator rows;
-// it runs over the slots that occur in the block and over K in steps of 32
-// bytes.  Per step, the operator slab (128 rows x 32 B x 4 digits, stored in
-// the MMA's canonical layout: one bulk copy) and the 128 sources' moment
-// digits (gathered rows) go to shared memory, and one thread issues ten
-// tcgen05.mma (M = 128 operator rows, N = 128 target rows, K = 32) into four
-// int32 accumulators: the 512 columns of tensor memory.  An MMA costs the
-// same whatever N (measured: 152 cycles for M = 128, K = 32, N = 32..256), so
-// N is the widest the accumulators allow.
+// octants of a region adjacent, so blocks that run together share sources.
+// A work item is a row block and 128 operator rows; it runs over the slots that
+// occur in the block and over K in steps of 32 bytes.  Per step, the operator
+// slab (128 rows x 32 B x 4 digits, stored in the MMA's canonical layout: one
+// bulk copy) and the 128 sources' moment digits (gathered 128-byte rows) go to
+// shared memory, and one thread issues ten tcgen05.mma (M = 128 operator rows,
+// N = 128 target rows, K = 32; 64 cycles each, measured back to back) into
+// four int32 accumulators: the 512 columns of tensor memory.
+//
+// Shared rows (p >= 7, i8_ops.h).  The field local and the potential local of
+// a coefficient take the same operator entries for source orders < p.  One
+// set of (p+2)^2 rows runs over those orders (phase 0), the field local is
+// read, order p alone is added (phase 1) and the potential local is read.  The
+// two rows of a coefficient have the same beta (checked when the tables are
+// built), so the digits, the sums and the results are those of separate rows.
+//
+// What bounds it (16M uniform points, p = 12, 35,000 steps an SM): separate
+// rows and the rows copied a thread per row took 44 ms, 1500 cycles a step
+// whatever the MMAs.  Copies of whole 128-byte lines (eight lanes a row, into
+// the 128-byte swizzle), arrivals by the copies themselves, the proxy fence in
+// a thread of its own and two K steps per set of barrier waits brought a step
+// to 995 cycles (shared rows: 18 instead of 12 steps a slot), 19.3 ms, against
+// 640 cycles of MMA.  TMA gathers of the rows (tile::gather4) took 2450 cycles
+// a step.  1M Plummer points, p = 10: 7.1 -> 3.8 ms.
 //
 // Roles (one block per SM, persistent over the items): warps 0-3 gather the
-// moment rows (cp.async) and issue the operator bulk copies; warp 8 allocates
-// tensor memory and issues the MMAs; warps 4-7, one per 32-lane quarter of
-// tensor memory, convert the sums and write the locals.  Shared-memory stages
-// and the accumulator pass between them through mbarriers; every wait is
-// bounded: on expiry the block records an error, stops its roles, waits for
-// its MMAs and copies and frees tensor memory (the host reports
-// FMM_ERR_TIMEOUT).
+// moment rows (cp.async) and issue the operator bulk copies; the relay thread
+// passes landed rows to the MMA's proxy; the MMA warp allocates tensor memory
+// and issues the MMAs; the epilogue warps, two per 32-lane quarter of tensor
+// memory, convert the sums and write the locals.  Shared-memory stages and the
+// accumulator pass between them through mbarriers; every wait is bounded: on
+// expiry the block records an error, stops its roles, waits for its MMAs and
+// copies and frees tensor memory (the host reports FMM_ERR_TIMEOUT).
 #include "eval_util.cuh"
 #include "i8_ops.h"
 
 #include <cub/device/device_radix_sort.cuh>
 
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <map>
@@ -69,9 +85,10 @@ namespace sfmm {
 
 constexpr int kI8Slots = 216;
 constexpr int kI8M = 128;                 // operator rows per item (MMA M, tensor-memory lanes)
-constexpr int kI8Stages = 6;
-constexpr int kI8Lag = 4;                 // gather stages in flight per producer thread
-constexpr int kI8Threads = 9 * 32;
+constexpr int kI8Steps = 2;               // K steps per pipeline stage: one set of barrier waits per 20 MMAs
+constexpr int kI8Stages = 3;
+constexpr int kI8EpiWarps = 8;
+constexpr int kI8Threads = (4 + kI8EpiWarps + 2) * 32;
 constexpr long kI8Spin = 1L << 22;        // mbarrier polls before a wait gives up
 
 // ND digits per value: N target rows per item (ND accumulators of N columns
@@ -79,16 +96,21 @@ constexpr long kI8Spin = 1L << 22;        // mbarrier polls before a wait gives 
 // The plans use ND = 4.
 template<int ND>
 struct I8Cfg {
-    static constexpr int N = ND == 3 ? 160 : 128;
+    static constexpr int N = 128;
+    static_assert(ND * N <= 512, "the accumulators fill tensor memory");
     static constexpr int OpSlab = ND * kI8M * 32;
     static constexpr int MdSlab = ND * N * 32;
-    static constexpr size_t Smem = size_t(kI8Stages) * (OpSlab + MdSlab);
+    static constexpr size_t Smem = size_t(kI8Stages) * kI8Steps * (OpSlab + MdSlab) + 1024;   // rounded up to 1024 in the kernel
 };
 
 struct I8DevTables {
     DevBuf<int8_t> op;       // [343 offsets][chunks][K steps][digit][128 rows x 32 B, canonical]
     DevBuf<double> beta;     // per operator row
     int R = 0, RA = 0, NCH = 0, KS = 0, ND = 4;
+    // shared rows (i8_shared_rows): R = (p + 2)^2 rows serve both locals; the
+    // first KB K steps hold source orders < p, the last one order p
+    bool shared = false;
+    int KB = 0;
 };
 
 struct I8PlanData {
@@ -125,10 +147,15 @@ __global__ void k_i8_beta(DirectArgs t, int p, int RA, int R, int KP, uint32_t* 
     if ((threadIdx.x & 31) == 0) atomicMax(beta_bits + r, __float_as_uint(mx));
 }
 
+// Operator digits.  shared: row r is the field local's row r; its columns of
+// source order p (which the field local does not take) hold the potential
+// local's entries of the same coefficient, rows r < RA only.  beta_bits
+// starts with the potential local's RA rows.
 template<int ND>
-__global__ void k_i8_opdigits(DirectArgs t, int p, int RA, int R, int NCH, int KS, const uint32_t* __restrict__ beta_bits,
-                              int8_t* __restrict__ op, double* __restrict__ beta)
+__global__ void k_i8_opdigits(DirectArgs t, int p, int RA, int R, int NCH, int KS, int shared,
+                              const uint32_t* __restrict__ beta_bits, int8_t* __restrict__ op, double* __restrict__ beta)
 {
+    const int KB = shared ? KS - 1 : KS, ro = shared ? RA : 0;
     const int KP = 32 * KS;
     const int64_t total = int64_t(343) * NCH * kI8M * KP;
     for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < total; e += int64_t(gridDim.x) * blockDim.x) {
@@ -138,15 +165,17 @@ __global__ void k_i8_opdigits(DirectArgs t, int p, int RA, int R, int NCH, int K
         const int c = static_cast<int>(e / (int64_t(KP) * kI8M * NCH));
         const int r = ch * kI8M + rr;
         int8_t d[ND] = {};
-        if (r < R && offset_valid(c)) {
-            const double b = double(__uint_as_float(beta_bits[r]));
+        const int kr = i8_column(k, p, KB, shared);
+        if (r < R && kr >= 0 && offset_valid(c)) {
+            const double b = double(__uint_as_float(beta_bits[ro + r]));
             int n, m, pi;
-            real_nm(k, n, m, pi);
-            if (b > 0) split_digits<ND>(op_entry(t, p, RA, c, r, k) * i8_gamma(n) / b, d);
+            real_nm(kr, n, m, pi);
+            const int row = shared && n == p ? (r < RA ? r : -1) : ro + r;
+            if (b > 0 && row >= 0) split_digits<ND>(op_entry(t, p, RA, c, row, kr) * i8_gamma(n) / b, d);
         }
         int8_t* slab = op + ((int64_t(c) * NCH + ch) * KS + k / 32) * I8Cfg<ND>::OpSlab;
         for (int i = 0; i < ND; ++i) slab[i * (kI8M * 32) + canon_off(rr, k % 32)] = d[i];
-        if (c == 0 && k == 0 && r < R) beta[r] = double(__uint_as_float(beta_bits[r]));
+        if (c == 0 && k == 0 && r < R) beta[r] = double(__uint_as_float(beta_bits[ro + r]));
     }
 }
 
@@ -315,8 +344,9 @@ __global__ void k_i8_alpha(EvalArgs a, uint32_t* __restrict__ alpha_bits)
 
 // moment digits of every node of levels >= 2 (warp per node and component)
 template<int ND>
-__global__ void k_i8_mdigits(EvalArgs a, int KS, const uint32_t* __restrict__ alpha_bits, int8_t* __restrict__ md)
+__global__ void k_i8_mdigits(EvalArgs a, int KS, int shared, const uint32_t* __restrict__ alpha_bits, int8_t* __restrict__ md)
 {
+    const int KB = shared ? KS - 1 : KS;
     __shared__ I8Scales sc;
     fill_scales(a, sc);
     const int lane = threadIdx.x & 31, qd = a.qdim, T = a.T, p = a.p, KP = 32 * KS;
@@ -331,9 +361,10 @@ __global__ void k_i8_mdigits(EvalArgs a, int KS, const uint32_t* __restrict__ al
         int8_t* dst = md + (g * qd + c) * int64_t(KS) * (32 * ND);
         for (int k = lane; k < KP; k += 32) {
             int8_t d[ND] = {};
-            if (k < (p + 1) * (p + 1) && al > 0) {
+            const int kr = i8_column(k, p, KB, shared);
+            if (kr >= 0 && al > 0) {
                 int n, m, im;
-                real_nm(k, n, m, im);
+                real_nm(kr, n, m, im);
                 const cplx v = a.M[(g * qd + c) * T + n * (n + 1) / 2 + m];
                 split_digits<ND>((im ? v.im : v.re) * sc.pw[l][n] / sc.gm[n] / al, d);
             }
@@ -351,6 +382,14 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t saddr)
 {
     // no swizzle; leading (K) byte offset 128, stride (M/N) byte offset 256; descriptor version 1
     return uint64_t((saddr >> 4) & 0x3FFF) | uint64_t(128 >> 4) << 16 | uint64_t(256 >> 4) << 32 | uint64_t(1) << 46;
+}
+
+// Gathered moment rows: 128 bytes a row (ND digits of 32 bytes) in the 128-byte
+// swizzle (16-byte piece c of row r at c ^ (r % 8)), 8-row groups 1024 bytes
+// apart; digit j starts 32 j bytes into the row.
+__device__ __forceinline__ uint64_t sdesc_md(uint32_t saddr)
+{
+    return uint64_t((saddr >> 4) & 0x3FFF) | uint64_t(1) << 16 | uint64_t(1024 >> 4) << 32 | uint64_t(1) << 46 | uint64_t(2) << 61;
 }
 
 // kind::i8 instruction descriptor: S32 accumulator, signed A and B, both K-major
@@ -423,9 +462,17 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
                  : "memory");
 }
 
-__device__ __forceinline__ void cp16(void* dst, const void* src, bool valid)
+// 16-byte copy, zeros where bytes is 0
+__device__ __forceinline__ void cp16(uint32_t dst, const void* src, int bytes)
 {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(su32(dst)), "l"(src), "r"(valid ? 16 : 0) : "memory");
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+
+// Arrival of the calling thread on bar when all its cp.async so far have
+// landed (counted in the barrier's expected arrivals).
+__device__ __forceinline__ void cp_arrive(uint64_t* bar)
+{
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(su32(bar)) : "memory");
 }
 
 __device__ __forceinline__ void tld16(uint32_t taddr, uint32_t (&r)[16])
@@ -444,42 +491,60 @@ struct I8Args {
     const int32_t *slot_src, *used, *nused, *rb_tgt, *rb_info;
     int64_t nrb;
     int tpb, NCH, KS, RA, R;
+    int shared, KB, nch_run;              // shared rows; the row chunks of this evaluation's outputs
     int* err;
 };
 
 struct I8Smem {
-    uint64_t full[kI8Stages], empty[kI8Stages];
+    uint64_t full[kI8Stages], empty[kI8Stages], landed[kI8Stages];
     uint64_t tfull, tempty;
     uint32_t tbase;
     int abort;
-    long long nfilled;                    // stages the producers filled
+    long long nfilled;                    // stages the producers filled or began
 };
+
+// K steps of an item per slot: phase 0 (all of them, or with shared rows the
+// source orders < p), then phase 1 (order p, the potential local's rows).
+struct I8Phases {
+    int k0, k1;
+    bool read0, read1;                    // the sums are read after the phase
+};
+__device__ __forceinline__ I8Phases i8_phases(const EvalArgs& a, const I8Args& g, int ch)
+{
+    I8Phases f;
+    f.k0 = g.shared ? g.KB : g.KS;
+    f.read1 = g.shared && a.want_pot && ch * kI8M < g.RA;
+    f.k1 = f.read1 ? g.KS - g.KB : 0;
+    f.read0 = !g.shared || a.want_field;
+    return f;
+}
 
 template<int ND>
 __global__ void __launch_bounds__(kI8Threads, 1) k_m2l_i8(EvalArgs a, I8Args g)
 {
     using C = I8Cfg<ND>;
     constexpr int kN = C::N, kOpSlab = C::OpSlab, kMdSlab = C::MdSlab;
-    extern __shared__ __align__(1024) uint8_t sm_raw[];
+    extern __shared__ uint8_t sm_raw[];
     __shared__ I8Smem ctl;
-    uint8_t* opS = sm_raw;                                   // [stage][kOpSlab]
-    uint8_t* mdS = sm_raw + kI8Stages * kOpSlab;             // [stage][kMdSlab]
+    uint8_t* opS = sm_raw + ((1024 - (su32(sm_raw) & 1023)) & 1023);   // [stage][step][kOpSlab]; the swizzle wants 1024-byte groups
+    uint8_t* mdS = opS + kI8Stages * kI8Steps * kOpSlab;     // [stage][step][kMdSlab]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int qd = a.qdim, KS = g.KS, NCH = g.NCH, tpb = g.tpb;
-    const int64_t items = g.nrb * NCH;
+    const int qd = a.qdim, KS = g.KS, tpb = g.tpb;
+    const int64_t items = g.nrb * g.nch_run;
     volatile int* abort = &ctl.abort;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kI8Stages; ++s) {
-            bar_init(&ctl.full[s], 128 + 1);
+            bar_init(&ctl.full[s], 2);                        // operator slab issued (and landed), rows relayed
+            bar_init(&ctl.landed[s], 128);
             bar_init(&ctl.empty[s], 1);
         }
         bar_init(&ctl.tfull, 1);
-        bar_init(&ctl.tempty, 128);
+        bar_init(&ctl.tempty, 32 * kI8EpiWarps);
         ctl.abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 8) {
+    if (warp == 4 + kI8EpiWarps) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(su32(&ctl.tbase)));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
@@ -489,88 +554,153 @@ __global__ void __launch_bounds__(kI8Threads, 1) k_m2l_i8(EvalArgs a, I8Args g)
     const uint32_t tbase = ctl.tbase;
 
     if (warp < 4) {
-        // ---------------- producers: operator slab (bulk copy) + gathered moment rows
-        const int tp = threadIdx.x;
+        // ---------------- producers: operator slab (one bulk copy) and 32 moment rows per warp.  A copy
+        // instruction takes 4 whole 128-byte rows (eight lanes a row).  Lane r holds the source of the warp's row
+        // r; the sources of the next slot are loaded one slot ahead, the slot list two ahead.
+        static_assert(ND == 4, "a moment row is one 128-byte line");
         int64_t n = 0;                                        // stages filled by this block
         bool ok = true;
+        const int piece = lane & 7, sub = lane >> 3;
         for (int64_t it = blockIdx.x; it < items && ok; it += gridDim.x) {
-            const int64_t rb = it / NCH;
-            const int ch = static_cast<int>(it % NCH);
+            const int64_t rb = it / g.nch_run;
+            const int ch = static_cast<int>(it % g.nch_run);
             const int info = g.rb_info[rb];
             const int oct = (info >> 8) & 7, ntg = info >> 12;
             const int cx = oct & 1, cy = (oct >> 1) & 1, cz = oct >> 2;
-            const int nst = g.nused[rb] * KS;
-            for (int st = 0; st < nst; ++st, ++n) {
-                const int s = static_cast<int>(n % kI8Stages);
-                const uint32_t ph = static_cast<uint32_t>(n / kI8Stages) & 1;
-                if (!bar_wait(&ctl.empty[s], ph ^ 1, abort)) {
-                    ok = false;
-                    break;
-                }
-                const int slot = g.used[rb * kI8Slots + st / KS], ks = st % KS;
-                const int dx = slot % 6 - 2 - cx, dy = (slot / 6) % 6 - 2 - cy, dz = slot / 36 - 2 - cz;
-                const int c = (dx + 3) + 7 * (dy + 3) + 49 * (dz + 3);
-                if (tp == 0) {
-                    bar_arrive_tx(&ctl.full[s], kOpSlab);
-                    bulk_g2s(opS + s * kOpSlab, g.op + ((int64_t(c) * NCH + ch) * KS + ks) * kOpSlab, kOpSlab, &ctl.full[s]);
-                }
-                uint8_t* dst = mdS + s * kMdSlab;
-                for (int row = tp; row < kN; row += 128) {
-                    const int t = row / qd, comp = row % qd;
-                    const int src = t < ntg ? g.slot_src[(rb * kI8Slots + slot) * tpb + t] : -1;
-                    const int8_t* sp = g.md + ((int64_t(src < 0 ? 0 : src) * qd + comp) * KS + ks) * (32 * ND);
-                    const int ro = (row >> 3) * 256 + (row & 7) * 16;
+            const int ns = g.nused[rb];
+            const I8Phases f = i8_phases(a, g, ch);
+            const int32_t* used = g.used + rb * kI8Slots;
+            const int row = warp * 32 + lane, comp = row % qd;
+            const bool has = row / qd < ntg;
+            const int32_t* tab = g.slot_src + rb * kI8Slots * tpb + (has ? row / qd : 0);
+            for (int ph = 0; ph < 2 && ok; ++ph) {
+                const int kn = ph ? f.k1 : f.k0, kb = ph ? g.KB : 0;
+                if (kn == 0 || ns == 0) continue;
+                int slot = used[0], slot1 = ns > 1 ? used[1] : 0;
+                int src = has ? tab[slot * tpb] : -1;
+                const int nst = ns * kn;
+                int st = 0;                                   // K step of the phase
+                for (int si = 0; si < ns && ok; ++si) {
+                    const int nsrc = has && si + 1 < ns ? tab[slot1 * tpb] : -1;
+                    const int slot2 = si + 2 < ns ? used[si + 2] : 0;
+                    const int dx = slot % 6 - 2 - cx, dy = (slot / 6) % 6 - 2 - cy, dz = slot / 36 - 2 - cz;
+                    const int c = (dx + 3) + 7 * (dy + 3) + 49 * (dz + 3);
+                    // first K step's moment row of the source, -1: none (the row is filled with zeros)
+                    const int mrow = src < 0 ? -1 : (src * qd + comp) * KS;
+                    const int8_t* from[8];
+                    int bytes[8];
 #pragma unroll
-                    for (int i = 0; i < ND; ++i) {
-                        cp16(dst + i * (kN * 32) + ro, sp + i * 32, src >= 0);
-                        cp16(dst + i * (kN * 32) + ro + 128, sp + i * 32 + 16, src >= 0);
+                    for (int i = 0; i < 8; ++i) {
+                        const int m = __shfl_sync(0xffffffffu, mrow, 4 * i + sub);
+                        from[i] = g.md + (int64_t(m < 0 ? 0 : m) + kb) * (32 * ND) + piece * 16;
+                        bytes[i] = m < 0 ? 0 : 16;
                     }
+                    for (int ks = kb; ks < kb + kn; ++ks, ++st) {
+                        const int s = static_cast<int>(n % kI8Stages), h = st % kI8Steps;
+                        if (h == 0) {
+                            if (!bar_wait(&ctl.empty[s], (static_cast<uint32_t>(n / kI8Stages) & 1) ^ 1, abort)) {
+                                ok = false;
+                                break;
+                            }
+                            if (threadIdx.x == 0) bar_arrive_tx(&ctl.full[s], kOpSlab * min(kI8Steps, nst - st));
+                        }
+                        const int u = s * kI8Steps + h;
+                        if (threadIdx.x == 0) {
+                            bulk_g2s(opS + u * kOpSlab, g.op + ((int64_t(c) * g.NCH + ch) * KS + ks) * kOpSlab, kOpSlab,
+                                     &ctl.full[s]);
+                        }
+                        const uint32_t dst = su32(mdS + u * kMdSlab + warp * (32 * 32 * ND) + sub * (32 * ND));
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            // row 4 i + sub of the warp: 16-byte piece at piece ^ (row % 8)
+                            cp16(dst + i * (4 * 32 * ND) + ((piece ^ (4 * (i & 1) + sub)) << 4), from[i], bytes[i]);
+                            from[i] += 32 * ND;
+                        }
+                        if (h == kI8Steps - 1 || st == nst - 1) {
+                            // arrives by itself once this thread's copies have landed
+                            cp_arrive(&ctl.landed[s]);
+                            ++n;
+                        }
+                    }
+                    slot = slot1;
+                    slot1 = slot2;
+                    src = nsrc;
+                    ok = __all_sync(0xffffffffu, ok);         // the next slot's shuffles take the whole warp
                 }
-                asm volatile("cp.async.commit_group;" ::: "memory");
-                // the stage issued kI8Lag steps ago has landed: publish it to the MMA (async proxy)
-                asm volatile("cp.async.wait_group %0;" ::"n"(kI8Lag) : "memory");
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                if (n >= kI8Lag) bar_arrive(&ctl.full[(n - kI8Lag) % kI8Stages]);
             }
         }
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        for (int64_t m = n - kI8Lag < 0 ? 0 : n - kI8Lag; m < n; ++m) bar_arrive(&ctl.full[m % kI8Stages]);
-        if (tp == 0) ctl.nfilled = n;
-    } else if (warp == 8) {
-        // ---------------- MMA issue (one thread)
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        if (threadIdx.x == 0) ctl.nfilled = n;                // a phase cut short by an abort left no stage half filled
+    } else if (warp == 5 + kI8EpiWarps) {
+        // ---------------- relay: a landed stage's rows, written through the generic proxy, become visible to the
+        // MMA's (async) proxy.  One thread of its own: in the MMA thread the fence delayed every step's issue.
         if (lane == 0) {
-            int64_t n = 0, nb = 0;
+            int64_t n = 0;
             bool ok = true;
             for (int64_t it = blockIdx.x; it < items && ok; it += gridDim.x) {
-                const int64_t rb = it / NCH;
-                const int nst = g.nused[rb] * KS;
-                if (nst == 0) continue;
-                if (!bar_wait(&ctl.tempty, (static_cast<uint32_t>(nb) & 1) ^ 1, abort)) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                for (int st = 0; st < nst; ++st, ++n) {
+                const I8Phases f = i8_phases(a, g, static_cast<int>(it % g.nch_run));
+                const int ns = g.nused[it / g.nch_run];
+                const int stages = (ns * f.k0 + kI8Steps - 1) / kI8Steps + (ns * f.k1 + kI8Steps - 1) / kI8Steps;
+                for (int st = 0; st < stages; ++st, ++n) {
                     const int s = static_cast<int>(n % kI8Stages);
-                    const uint32_t ph = static_cast<uint32_t>(n / kI8Stages) & 1;
-                    if (!bar_wait(&ctl.full[s], ph, abort)) {
+                    if (!bar_wait(&ctl.landed[s], static_cast<uint32_t>(n / kI8Stages) & 1, abort)) {
                         ok = false;
                         break;
                     }
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t ao = su32(opS + s * kOpSlab), bo = su32(mdS + s * kMdSlab);
-                    // products of operator digit i and moment digit j of weight 2^-8(i+j) >= 2^-8(ND-1),
-                    // summed into accumulator i + j; the first of each accumulator in an item overwrites it
-#pragma unroll
-                    for (int gsum = 0; gsum < ND; ++gsum)
-#pragma unroll
-                        for (int i = 0; i <= gsum; ++i)
-                            mma_i8<kN>(tbase + gsum * kN, sdesc(ao + i * (kI8M * 32)), sdesc(bo + (gsum - i) * (kN * 32)),
-                                       (st > 0 || i > 0) ? 1u : 0u);
-                    mma_commit(&ctl.empty[s]);
+                    bar_arrive(&ctl.full[s]);
                 }
-                if (!ok) break;
-                mma_commit(&ctl.tfull);
-                ++nb;
+            }
+        }
+        __syncwarp();
+    } else if (warp == 4 + kI8EpiWarps) {
+        // ---------------- MMA issue (one thread)
+        if (lane == 0) {
+            int64_t n = 0, nb = 0;                            // stages consumed; readings of the sums asked for
+            bool ok = true;
+            for (int64_t it = blockIdx.x; it < items && ok; it += gridDim.x) {
+                const int64_t rb = it / g.nch_run;
+                const I8Phases f = i8_phases(a, g, static_cast<int>(it % g.nch_run));
+                const int ns = g.nused[rb];
+                if (ns == 0) continue;
+                bool fresh = true;                            // the item's first step overwrites the sums
+                for (int ph = 0; ph < 2 && ok; ++ph) {
+                    const int nst = ns * (ph ? f.k1 : f.k0);
+                    if (nst == 0) continue;
+                    // every reading asked for so far is done
+                    if (!bar_wait(&ctl.tempty, (static_cast<uint32_t>(nb) & 1) ^ 1, abort)) {
+                        ok = false;
+                        break;
+                    }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    for (int st = 0; st < nst; st += kI8Steps, ++n) {
+                        const int s = static_cast<int>(n % kI8Stages);
+                        if (!bar_wait(&ctl.full[s], static_cast<uint32_t>(n / kI8Stages) & 1, abort)) {
+                            ok = false;
+                            break;
+                        }
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        // products of operator digit i and moment digit j of weight 2^-8(i+j) >= 2^-8(ND-1),
+                        // summed into accumulator i + j; a fresh item's first product of each overwrites it
+                        for (int h = 0; h < kI8Steps && st + h < nst; ++h) {
+                            const uint64_t da = sdesc(su32(opS + (s * kI8Steps + h) * kOpSlab));
+                            const uint64_t db = sdesc_md(su32(mdS + (s * kI8Steps + h) * kMdSlab));
+#pragma unroll
+                            for (int gsum = 0; gsum < ND; ++gsum)
+#pragma unroll
+                                for (int i = 0; i <= gsum; ++i)
+                                    mma_i8<kN>(tbase + gsum * kN, da + i * (kI8M * 32 / 16), db + (gsum - i) * (32 / 16),
+                                               fresh && i == 0 ? 0u : 1u);
+                            fresh = false;
+                        }
+                        mma_commit(&ctl.empty[s]);
+                    }
+                    if (!ok) break;
+                    if (ph ? f.read1 : f.read0) {
+                        mma_commit(&ctl.tfull);
+                        ++nb;
+                    }
+                }
             }
             if (!ok || *abort) {
                 // let the MMAs already issued finish before tensor memory is freed
@@ -580,76 +710,82 @@ __global__ void __launch_bounds__(kI8Threads, 1) k_m2l_i8(EvalArgs a, I8Args g)
         }
         __syncwarp();
     } else {
-        // ---------------- epilogue: lanes of quarter q = warp - 4 are operator rows
-        const int q = warp - 4;
+        // ---------------- epilogue: lanes of quarter q = warp % 4 are operator rows; two warps a quarter, half of
+        // the columns each (the MMAs wait meanwhile)
+        const int q = warp & 3, col0 = (warp - 4) / 4 * (kN * 4 / kI8EpiWarps);
         const int rl = q * 32 + lane;                         // tensor-memory lane = row in the item
         const int T = a.T, T1 = a.T1;
         int64_t nb = 0;
         bool ok = true;
         for (int64_t it = blockIdx.x; it < items && ok; it += gridDim.x) {
-            const int64_t rb = it / NCH;
-            const int ch = static_cast<int>(it % NCH);
+            const int64_t rb = it / g.nch_run;
+            const int ch = static_cast<int>(it % g.nch_run);
             const int info = g.rb_info[rb];
             const int l = info & 255, ntg = info >> 12;
-            const int nst = g.nused[rb] * KS;
+            const int ns = g.nused[rb];
+            const I8Phases f = i8_phases(a, g, ch);
             const int r = ch * kI8M + rl;
-            // this lane's output coefficient
-            bool on = r < g.R;
-            int j = 0, kk = 0, po = 0, isA = 1;
-            if (on) {
-                if (r < g.RA) {
-                    real_nm(r, j, kk, po);
+            for (int ph = 0; ph < 2; ++ph) {
+                if (!(ph ? f.read1 : f.read0)) continue;
+                // this lane's output coefficient.  Shared rows: the field local's after phase 0, the potential
+                // local's after phase 1; else rows r < RA are the potential local's
+                bool on, isA;
+                int j = 0, kk = 0, po = 0;
+                if (g.shared) {
+                    isA = ph == 1;
+                    on = r < (isA ? g.RA : g.R);
+                    if (on) real_nm(r, j, kk, po);
                 } else {
-                    real_nm(r - g.RA, j, kk, po);
-                    isA = 0;
+                    isA = r < g.RA;
+                    on = r < g.R && (isA ? a.want_pot : a.want_field);
+                    if (on) real_nm(isA ? r : r - g.RA, j, kk, po);
                 }
-                on = isA ? a.want_pot : a.want_field;
-            }
-            // alpha of the column's tree (a forest's members keep their own moment scales)
-            double scale = 0.0;
-            if (on && nst > 0) scale = g.beta[r] / (127.0 * 127.0) * pow(double(1 << l) / a.box->width, double(j + 1));
-            if (nst > 0) {
-                const bool got = bar_wait(&ctl.tfull, static_cast<uint32_t>(nb) & 1, abort);
-                if (!__all_sync(0xffffffffu, got)) {          // warp-uniform: the loads below are .aligned
-                    ok = false;
-                    break;
-                }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            }
-            const int tri_i = j * (j + 1) / 2 + kk;
-            double* base = on ? (isA ? &a.LA[0].re : &a.LB[0].re) : nullptr;
-            const int stride = isA ? T : T1;
-            for (int c0 = 0; c0 < kN; c0 += 16) {
-                uint32_t sg[ND][16];
-                if (nst > 0) {
-                    const uint32_t ta = tbase + (uint32_t(q * 32) << 16) + c0;
-#pragma unroll
-                    for (int gsum = 0; gsum < ND; ++gsum) tld16(ta + gsum * kN, sg[gsum]);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                }
-                if (!on) continue;
-#pragma unroll
-                for (int e = 0; e < 16; ++e) {
-                    const int col = c0 + e;
-                    const int t = col / qd, comp = col % qd;
-                    if (t >= ntg || t >= tpb) continue;
-                    const int64_t node = g.rb_tgt[rb * tpb + t];
-                    double v = 0.0;
-                    if (nst > 0) {
-#pragma unroll
-                        for (int gsum = ND - 1; gsum >= 0; --gsum) v = v * (1.0 / 256) + double(int(sg[gsum][e]));
-                        const int tr = a.node_tree ? a.node_tree[node] : 0;
-                        v *= scale * double(__uint_as_float(g.alpha[tr * (kKeyLevel + 2) + l]));
+                // alpha of the column's tree (a forest's members keep their own moment scales)
+                double scale = 0.0;
+                if (on && ns > 0) scale = g.beta[r] / (127.0 * 127.0) * pow(double(1 << l) / a.box->width, double(j + 1));
+                if (ns > 0) {
+                    const bool got = bar_wait(&ctl.tfull, static_cast<uint32_t>(nb) & 1, abort);
+                    if (!__all_sync(0xffffffffu, got)) {          // warp-uniform: the loads below are .aligned
+                        ok = false;
+                        break;
                     }
-                    double* dst = base + 2 * ((node * qd + comp) * stride + tri_i);
-                    dst[po] = v;
-                    if (kk == 0) dst[1] = 0.0;               // Im of an m = 0 coefficient
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 }
-            }
-            if (nst > 0) {
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                bar_arrive(&ctl.tempty);
-                ++nb;
+                const int tri_i = j * (j + 1) / 2 + kk;
+                double* base = on ? (isA ? &a.LA[0].re : &a.LB[0].re) : nullptr;
+                const int stride = isA ? T : T1;
+                for (int c0 = col0; c0 < col0 + kN * 4 / kI8EpiWarps; c0 += 16) {
+                    uint32_t sg[ND][16];
+                    if (ns > 0) {
+                        const uint32_t ta = tbase + (uint32_t(q * 32) << 16) + c0;
+#pragma unroll
+                        for (int gsum = 0; gsum < ND; ++gsum) tld16(ta + gsum * kN, sg[gsum]);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    }
+                    if (!on) continue;
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) {
+                        const int col = c0 + e;
+                        const int t = col / qd, comp = col % qd;
+                        if (t >= ntg || t >= tpb) continue;
+                        const int64_t node = g.rb_tgt[rb * tpb + t];
+                        double v = 0.0;
+                        if (ns > 0) {
+#pragma unroll
+                            for (int gsum = ND - 1; gsum >= 0; --gsum) v = v * (1.0 / 256) + double(int(sg[gsum][e]));
+                            const int tr = a.node_tree ? a.node_tree[node] : 0;
+                            v *= scale * double(__uint_as_float(g.alpha[tr * (kKeyLevel + 2) + l]));
+                        }
+                        double* dst = base + 2 * ((node * qd + comp) * stride + tri_i);
+                        dst[po] = v;
+                        if (kk == 0) dst[1] = 0.0;               // Im of an m = 0 coefficient
+                    }
+                }
+                if (ns > 0) {
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    bar_arrive(&ctl.tempty);
+                    ++nb;
+                }
             }
         }
     }
@@ -657,13 +793,13 @@ __global__ void __launch_bounds__(kI8Threads, 1) k_m2l_i8(EvalArgs a, I8Args g)
     __syncthreads();
     if (ctl.abort && threadIdx.x == 0) {
         atomicExch(g.err, 1);
-        // operator copies into stages the MMA may not have consumed land before shared memory is released
+        // copies into stages the MMA may not have consumed land before shared memory is released
         const long long n = ctl.nfilled;
         for (long long m = n - kI8Stages < 0 ? 0 : n - kI8Stages; m < n; ++m)
             bar_drain(&ctl.full[m % kI8Stages], static_cast<uint32_t>(m / kI8Stages) & 1);
     }
     __syncthreads();
-    if (warp == 8) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tbase));
+    if (warp == 4 + kI8EpiWarps) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tbase));
 }
 
 }  // namespace
@@ -679,20 +815,27 @@ static std::shared_ptr<I8DevTables> i8_tables_on_device(int device, int p, int N
     auto dt = direct_tables_on_device(device, p, st);
     auto t = std::make_shared<I8DevTables>();
     t->RA = (p + 1) * (p + 1);
-    t->R = t->RA + (p + 2) * (p + 2);
-    t->NCH = rdiv_up(t->R, kI8M);
-    t->KS = rdiv_up((p + 1) * (p + 1), 32);
-    const int KP = 32 * t->KS;
+    const int RAB = t->RA + (p + 2) * (p + 2);
     DirectArgs da{dt->coef.ptr, dt->ncoef, dt->zil.ptr, dt->nz, reinterpret_cast<const cplx*>(dt->eil2.ptr), dt->ne};
     DevBuf<uint32_t> bb;
-    bb.alloc(t->R, st);
+    bb.alloc(RAB, st);
     SFMM_CUDA(cudaMemsetAsync(bb.ptr, 0, bb.bytes(), st));
-    k_i8_beta<<<t->R, 256, 0, st>>>(da, p, t->RA, t->R, KP, bb.ptr);
+    k_i8_beta<<<RAB, 256, 0, st>>>(da, p, t->RA, RAB, t->RA, bb.ptr);
     SFMM_CHECK_LAUNCH();
+    // both locals in one set of rows where that takes fewer MMAs and each
+    // coefficient's two rows have one scale: its digits are then the same numbers
+    std::vector<uint32_t> hb(RAB);
+    SFMM_CUDA(cudaMemcpyAsync(hb.data(), bb.ptr, bb.bytes(), cudaMemcpyDeviceToHost, st));
+    SFMM_CUDA(cudaStreamSynchronize(st));
+    t->shared = i8_shared_rows(p) && std::equal(hb.begin(), hb.begin() + t->RA, hb.begin() + t->RA);
+    t->R = t->shared ? RAB - t->RA : RAB;
+    t->KB = rdiv_up(p * p, 32);
+    t->KS = t->shared ? t->KB + 1 : rdiv_up(t->RA, 32);
+    t->NCH = rdiv_up(t->R, kI8M);
     t->ND = ND;
     t->op.alloc(size_t(343) * t->NCH * t->KS * ND * kI8M * 32, st);
     t->beta.alloc(t->R, st);
-    k_i8_opdigits<4><<<2048, 256, 0, st>>>(da, p, t->RA, t->R, t->NCH, t->KS, bb.ptr, t->op.ptr, t->beta.ptr);
+    k_i8_opdigits<4><<<2048, 256, 0, st>>>(da, p, t->RA, t->R, t->NCH, t->KS, t->shared, bb.ptr, t->op.ptr, t->beta.ptr);
     SFMM_CHECK_LAUNCH();
     SFMM_CUDA(cudaStreamSynchronize(st));
     slot = t;
@@ -806,15 +949,17 @@ void launch_m2l_i8(Plan& pl, const EvalArgs& a, cudaStream_t st)
     const unsigned gw = static_cast<unsigned>(std::min<int64_t>(rows / 8 + 1, int64_t(sms) * 16));
     k_i8_alpha<<<gw, 256, 0, st>>>(a, d.alpha.ptr);
     SFMM_CHECK_LAUNCH();
-    k_i8_mdigits<4><<<gw, 256, 0, st>>>(a, tb.KS, d.alpha.ptr, d.md.ptr);
+    k_i8_mdigits<4><<<gw, 256, 0, st>>>(a, tb.KS, tb.shared, d.alpha.ptr, d.md.ptr);
     SFMM_CHECK_LAUNCH();
+    // with shared rows the potential alone needs only the chunks that hold its RA rows
+    const int nch_run = tb.shared && !a.want_field ? rdiv_up(tb.RA, kI8M) : tb.NCH;
     I8Args g{tb.op.ptr, tb.beta.ptr, d.md.ptr, d.alpha.ptr, d.slot_src.ptr, d.used.ptr, d.nused.ptr, d.rb_tgt.ptr,
-             d.rb_info.ptr, d.nrb, d.tpb, tb.NCH, tb.KS, tb.RA, tb.R, a.wait_err};
+             d.rb_info.ptr, d.nrb, d.tpb, tb.NCH, tb.KS, tb.RA, tb.R, tb.shared, tb.KB, nch_run, a.wait_err};
     static std::once_flag attr;
     std::call_once(attr, [] {
         SFMM_CUDA(cudaFuncSetAttribute(k_m2l_i8<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(I8Cfg<4>::Smem)));
     });
-    const int64_t items = d.nrb * tb.NCH;
+    const int64_t items = d.nrb * nch_run;
     const unsigned grid = static_cast<unsigned>(std::max<int64_t>(std::min<int64_t>(items, sms), 1));
     k_m2l_i8<4><<<grid, kI8Threads, I8Cfg<4>::Smem, st>>>(a, g);
     SFMM_CHECK_LAUNCH();

@@ -102,7 +102,7 @@ size_t estimate_bytes(int64_t n, int p, int qdim, int leaf, int precision)
     // mixed plans' tensor-core M2L (m2l_i8.cu): slot table, block lists and
     // four digits of the padded real moments per node
     if (precision == FMM_PRECISION_MIXED && p <= sfmm::kI8MaxOrder)
-        per_node += 216 * 4 + 16 + 4.0 * 32 * ((p + 1) * (p + 1) / 32 + 1) * qdim;
+        per_node += 216 * 4 + 16 + 4.0 * 32 * ((p + 1) * (p + 1) / 32 + 2) * qdim;
     return static_cast<size_t>(per_point * double(n) + per_node * nodes + (64 << 20));
 }
 
