@@ -484,7 +484,7 @@ void plan_init(Plan& pl)
     pl.M.alloc(size_t(t.n_nodes) * pl.qdim * pl.T, st);
     pl.LA.alloc(size_t(t.n_nodes) * pl.qdim * pl.T, st);
     pl.LB.alloc(size_t(t.n_nodes) * pl.qdim * pl.T1, st);
-    if (pl.precision == FMM_PRECISION_MIXED) pl.m32.alloc(size_t(t.n_nodes) * pl.qdim * pl.T, st);
+    if (pl.precision == FMM_PRECISION_MIXED && pl.p >= kTf32MinOrder) pl.m32.alloc(size_t(t.n_nodes) * pl.qdim * pl.T, st);
     shift_setup(pl);
     p2p_setup(pl);
     pl.m2l_ctr.alloc(1, st);
@@ -503,6 +503,7 @@ void plan_init(Plan& pl)
     pl.out.alloc(size_t(t.n) * kmax, st);
     pl.out2.alloc(size_t(t.n) * kmax, st);
     m2l_i8_setup(pl);
+    m2l_tile_setup(pl);
 }
 
 static EvalArgs make_args(Plan& pl, double* pot, double* field)
@@ -659,7 +660,7 @@ void plan_evaluate(Plan& pl, const double* Q, double* pot, double* field, cudaEv
         SFMM_CUDA(cudaEventRecord(pl.ev[1], st));
         if (a.m2l_direct) launch_m2l_direct(a, t.lvl_off[1], t.lvl_off[t.depth], sms, st);
         else if (pl.i8) launch_m2l_i8(pl, a, st);
-        else launch_m2l(a, t.lvl_off[1], t.lvl_off[t.depth], sms, st);
+        else if (!launch_m2l_tile(pl, a, st)) launch_m2l(a, t.lvl_off[1], t.lvl_off[t.depth], sms, st);
         near_field();
         SFMM_CUDA(cudaEventRecord(pl.ev[2], st));
         const size_t head2 = (32 + 2 * 4 * (2 * kMaxOrder + 1) + 2 * 4 * (2 * kMaxOrder + 3)) * sizeof(double);
@@ -707,6 +708,7 @@ void plan_set_shard(Plan& pl, int index, int count)
     pl.own_parent_e.clear();
     if (count == 1) {
         pl.own_leaf.release();
+        m2l_tile_setup(pl);
         return;
     }
     // this shard's leaves, level by level, balanced by points (shard_ranges.h)
@@ -732,6 +734,7 @@ void plan_set_shard(Plan& pl, int index, int count)
         pl.own_parent_b.push_back(b + shard_begin(nq, count, index));
         pl.own_parent_e.push_back(b + shard_end(nq, count, index));
     }
+    m2l_tile_setup(pl);
 }
 
 void plan_evaluate_stage(Plan& pl, const double* Q, double* pot, double* field, int stage)
@@ -786,6 +789,7 @@ void plan_evaluate_stage(Plan& pl, const double* Q, double* pot, double* field, 
         }
         SFMM_CUDA(cudaMemsetAsync(pl.LA.ptr, 0, pl.LA.bytes(), st));
         SFMM_CUDA(cudaMemsetAsync(pl.LB.ptr, 0, pl.LB.bytes(), st));
+        if (!a.m2l_direct && launch_m2l_tile(pl, a, st)) return;
         for (int q = 1; q < t.depth; ++q) {
             if (a.m2l_direct) launch_m2l_direct(a, pl.own_parent_b[q], pl.own_parent_e[q], sms, st);
             else launch_m2l(a, pl.own_parent_b[q], pl.own_parent_e[q], sms, st);

@@ -84,6 +84,7 @@ struct EvalArgs {
     double* p2p_part;
     int* p2p_ctr;
     int* m2l_ctr;                         // FP64 M2L: the counter blocks take sibling groups from
+    const int32_t* m2l_list;              // group kernels: the parents to take (their indices are then the range); NULL = all
     int m2l_force_rows;                   // run the row-owner M2L kernel (plan made with SFMM_M2L_KERNEL=rows)
     const uint8_t* own_leaf;              // sharded plan: 1 for this shard's leaves (global leaf id); NULL = all
     const int32_t* node_tree;             // forest: member tree of each node; NULL = one tree
@@ -114,6 +115,7 @@ struct PlanTables {
     DevBuf<float> rf32, tz32, tzl32;
     int rf32_nf = 0, tz32_nf = 0;
     DevBuf<double> sh_unit;                 // M2M / L2L maps at rho = 1 (shift.cu)
+    DevBuf<double> tile_ops, tile_zero;     // tiled M2L (m2l_tile.cu): operators per class, a row of zero moments
 };
 
 // Direct-M2L tables of one order on one device (shared like PlanTables).
@@ -145,7 +147,17 @@ struct Plan {
     // near-field work items (p2p.cu, p2p_setup)
     DevBuf<int4> p2p_item;
     DevBuf<int32_t> p2p_row, p2p_parts, p2p_rowoff, p2p_ctr;
-    DevBuf<int32_t> m2l_ctr;                  // M2L group counter (m2l.cu)
+    DevBuf<int32_t> m2l_ctr;                  // M2L work counter (m2l.cu, m2l_tile.cu)
+    // tiled M2L (m2l_tile.cu): split parents by level, chunks of them, the blocks' slot tables
+    DevBuf<int32_t> mt_parent, mt_table;
+    DevBuf<int4> mt_chunk;
+    int64_t mt_chunks = 0;
+    int mt_tpb = 0, mt_warps = 0;
+    bool mt_on = false;                       // the plan takes the tiled M2L (mt_groups' parents apart)
+    bool mt_split = false;                    // the parts of a tile in blocks of their own
+    DevBuf<double2> mt_part;                  // their sums
+    DevBuf<int32_t> mt_group;                 // a forest's parents of sparse members: the group kernel takes them
+    int64_t mt_groups = 0;
     bool m2l_force_rows = false;              // SFMM_M2L_KERNEL=rows at plan creation
     int m2l_method = FMM_M2L_METHOD_ROTATION;        // fmm_plan_set_m2l
     // sharded evaluation (fmm_plan_set_shard): this plan's share of one solve
@@ -160,7 +172,7 @@ struct Plan {
     int64_t p2p_items = 0, p2p_rows = 0;
     DevBuf<double> qin, uio_pot, uio_field;   // staging for host pointers
     // M2M / L2L as matrix products (shift.cu): per children level the octant
-    // maps, compact slots of the parents that have children, scratch rows
+    // maps; compact slots of the parents that have children (levels >= 1)
     bool shift_on = false;
     DevBuf<double> sh_ops;
     DevBuf<int32_t> sh_slot, sh_list;
@@ -183,6 +195,20 @@ void build_unit_shift_ops(PlanTables& tab, int p, cudaStream_t st);
 void shift_setup(Plan& pl);
 void shift_m2m(Plan& pl, const EvalArgs& a, int lp, cudaStream_t st);
 void shift_l2l(Plan& pl, const EvalArgs& a, int lc, cudaStream_t st);
+// m2l_tile.cu: the FP64 M2L of orders kTileMinOrder..kTileMaxOrder; operators
+// per (device, p), set-up per plan (after shift_setup; again after
+// plan_set_shard), launch (false: the plan takes another kernel)
+constexpr int kTileMinOrder = 2, kTileMaxOrder = 12;
+constexpr int kTf32MinOrder = 11;         // lowest order at which mixed plans use the TF32 M2L (m2l.cu)
+// targets (x charge components) below which a tile's parts run in blocks of their own
+constexpr int64_t kTileSplitRows = 24 * 1024;
+// parents from which on they are sorted by the pattern of their neighbours (25 us of set-up; 100,000 uniform points,
+// p = 8, 585 parents: M2L 0.81 -> 0.72 ms)
+constexpr int64_t kTileSortMin = 512;
+void build_tile_ops(PlanTables& tb, int P, cudaStream_t st);
+bool m2l_tile_supported(const Plan& pl);
+void m2l_tile_setup(Plan& pl);
+bool launch_m2l_tile(Plan& pl, const EvalArgs& a, cudaStream_t st);
 // p2p.cu: near-field work items of the plan's tree (leaves with a large near
 // field split into parts), built at plan creation
 void p2p_setup(Plan& pl);

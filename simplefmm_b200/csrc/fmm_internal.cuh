@@ -240,7 +240,18 @@ struct Tree {
     DevBuf<int32_t> node_tree;
     int n_trees = 1;
     std::vector<double> member_width;     // root-cube width of each member
+    std::vector<uint8_t> member_sparse;   // m2l_sparse of each member
+    std::vector<int64_t> member_node;     // first node of member r at level l: [l (members + 1) + r]
 };
+
+// Whether a tree's interaction lists are too short for the tiled FP64 M2L, whose
+// tiles run over every offset that some target of theirs has (m2l_tile.cu):
+// surfaces have ~40 sources a target, volumes 90 to 160.  Measured, tiled
+// against group kernel (M2L, p = 10): shell 20k points (39 a target) 0.53 / 0.38
+// ms, 400k (42) 3.5 / 2.8; Plummer 20k (90) 0.59 / 1.06, 400k (150) 4.5 / 7.2.
+// Trees of a few hundred targets are latency-bound and faster tiled: shell
+// 3,000 points (26) 0.24 / 0.27, uniform 3,000 (38) 0.25 / 0.30.
+inline bool m2l_sparse(int64_t pairs, int64_t targets) { return targets >= 1024 && pairs < 56 * targets; }
 
 struct Plan;
 

@@ -257,6 +257,19 @@ void build_forest(Tree& F, const std::vector<const Tree*>& members)
     F.n_trees = B;
     F.member_width.resize(B);
     for (int r = 0; r < B; ++r) F.member_width[r] = mv[r].width;
+    F.member_sparse.resize(B);
+    for (int r = 0; r < B; ++r) {
+        const Tree& t = *members[r];
+        F.member_sparse[r] = m2l_sparse(t.il_nnz, t.depth >= 2 ? t.n_nodes - t.lvl_off[2] : 0);
+    }
+    F.member_node.resize(size_t(F.depth + 1) * (B + 1));
+    for (int l = 0; l <= F.depth; ++l) {
+        int64_t o = F.lvl_off[l];
+        for (int r = 0; r <= B; ++r) {
+            F.member_node[size_t(l) * (B + 1) + r] = o;
+            if (r < B && l <= members[r]->depth) o += members[r]->lvl_off[l + 1] - members[r]->lvl_off[l];
+        }
+    }
     F.leaf_node.alloc(nl, st);
     DevBuf<int32_t> ilcnt, nrcnt;
     ilcnt.alloc(nn + 1, st);

@@ -39,7 +39,6 @@ namespace {
 constexpr int kCB = 4;                    // columns per batch
 constexpr int kMaxGroupPairs = 8 * 189;   // <= 8 siblings x n_ilist_max (partition.hpp:149)
 constexpr int kNumClasses = 70;           // fmm.hpp:169
-constexpr int kTf32MinOrder = 11;         // lowest order at which mixed plans use the TF32 M2L
 
 template<int P>
 struct RowCfg {
@@ -122,7 +121,8 @@ __global__ void __launch_bounds__(RowCfg<P>::NT) k_m2l_rows(EvalArgs a, int64_t 
     double Pr[P + 1], Qr[P + 1], PBr[P + 2], QBr[P + 2];
     int cls_b = -1, cls_d = -1;
 
-    for (int64_t g = g0 + blockIdx.x; g < g1; g += gridDim.x) {
+    for (int64_t gi = g0 + blockIdx.x; gi < g1; gi += gridDim.x) {
+        const int64_t g = a.m2l_list ? a.m2l_list[gi] : gi;
         const int nc = a.nchild[g];
         if (nc == 0) continue;
         const int cb = a.child_beg[g];
@@ -677,13 +677,16 @@ __global__ void __launch_bounds__(32 * NW, NW <= 8 ? (LEAN ? 4 : 3) : 1) k_m2l_m
     // children's interaction lists; the resident blocks stay busy to the end)
     __shared__ int64_t next_group;
     auto take = [&]() -> int64_t {
-        if (tid == 0) next_group = g0 + atomicAdd(a.m2l_ctr, 1);
+        if (tid == 0) {
+            const int64_t i = g0 + atomicAdd(a.m2l_ctr, 1);
+            next_group = i >= g1 ? -1 : a.m2l_list ? a.m2l_list[i] : i;
+        }
         __syncthreads();
         const int64_t g = next_group;
         __syncthreads();
         return g;
     };
-    for (int64_t g = take(); g < g1; g = take()) {
+    for (int64_t g = take(); g >= 0; g = take()) {
         const int nc = a.nchild[g];
         if (nc == 0) continue;
         const int cb = a.child_beg[g];
@@ -1603,11 +1606,13 @@ void launch_m2l_p(const EvalArgs& a, int64_t g0, int64_t g1, int sms, cudaStream
         launch_rows_fallback<P>(a, g0, g1, sms, st);
         return;
     }
-    if constexpr (P >= 2) {
+    if constexpr (P >= kTf32MinOrder) {
         // mixed plans take the TF32 kernel where it is the faster one (p = 12:
         // 281 ms against 364 ms on 16M uniform points; p = 10: 92 ms against
         // 81 ms on 4M Plummer points, where the FP64 kernel runs instead)
-        if (a.mixed && P >= kTf32MinOrder && try_launch_tf32<P>(a, g0, g1, sms, st)) return;
+        if (a.mixed && try_launch_tf32<P>(a, g0, g1, sms, st)) return;
+    }
+    if constexpr (P >= 2) {
         if (try_launch_mma<P, 1, 8, true>(a, g0, g1, sms, st)) return;
         if (try_launch_mma<P, 1, 8, false>(a, g0, g1, sms, st)) return;
     }
@@ -1618,16 +1623,19 @@ void launch_m2l_p(const EvalArgs& a, int64_t g0, int64_t g1, int sms, cudaStream
 
 void build_m2l_fragments(PlanTables& tb, int P, bool mixed, cudaStream_t st)
 {
+    if (P >= kTileMinOrder && P <= kTileMaxOrder) build_tile_ops(tb, P, st);
     tb.rfrag_nf = mma_foff(P + 2);
-    tb.rfrag.alloc(size_t(kNumClasses) * tb.rfrag_nf * 4 * 32, st);
-    const int nfz = std::max(tz_foff(P, P + 2), 1);
-    tb.tzfrag.alloc(size_t(nfz) * 32, st);
-    tb.tzl.alloc(size_t(P + 1) * (P + 2), st);
-    k_frag_rot<<<256, 256, 0, st>>>(tb.rot.ptr, tb.rot_off.ptr, tb.rot_len, P, tb.rfrag_nf, tb.rfrag.ptr);
-    SFMM_CHECK_LAUNCH();
-    k_frag_tz<<<16, 256, 0, st>>>(tb.tzx.ptr, tb.tzx_off.ptr, P, tz_foff(P, P + 2), tb.tzfrag.ptr, tb.tzl.ptr);
-    SFMM_CHECK_LAUNCH();
-    if (mixed) {
+    if (P >= 2) {
+        tb.rfrag.alloc(size_t(kNumClasses) * tb.rfrag_nf * 4 * 32, st);
+        const int nfz = std::max(tz_foff(P, P + 2), 1);
+        tb.tzfrag.alloc(size_t(nfz) * 32, st);
+        tb.tzl.alloc(size_t(P + 1) * (P + 2), st);
+        k_frag_rot<<<256, 256, 0, st>>>(tb.rot.ptr, tb.rot_off.ptr, tb.rot_len, P, tb.rfrag_nf, tb.rfrag.ptr);
+        SFMM_CHECK_LAUNCH();
+        k_frag_tz<<<16, 256, 0, st>>>(tb.tzx.ptr, tb.tzx_off.ptr, P, tz_foff(P, P + 2), tb.tzfrag.ptr, tb.tzl.ptr);
+        SFMM_CHECK_LAUNCH();
+    }
+    if (mixed && P >= kTf32MinOrder) {
         tb.rf32_nf = tf_foff(P + 2);
         tb.tz32_nf = std::max(tf_zoff(P, P + 2), 1);
         tb.rf32.alloc(size_t(kNumClasses) * tb.rf32_nf * 4 * 64 * 4, st);     // float4, high and low parts

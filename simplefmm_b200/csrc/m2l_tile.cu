@@ -1,0 +1,343 @@
+// FP64 M2L (fmm.hpp:620-688) for orders 2..12: rotate, translate along z,
+// rotate back, as FP64 tensor-core products (mma.sync m8n8k4 f64) over tiles of
+// targets that share every offset.
+//
+// Work decomposition.  All targets of one octant (position in the parent) at
+// one level have their sources at the same offsets d, so for a given d they
+// share the whole operator: rotation class, distance and azimuth.  A tile is
+// up to 32 columns (16 above p = 10): the children in one octant of up to 32
+// consecutive split parents of a level (a column is a target and a charge
+// component).  A block runs over the tile's slots (the offsets that occur, at
+// most 189 of the 6 x 6 x 6 box around the target); a target without a source
+// in a slot takes zero moments.  Every operator fragment read serves 4 MMAs
+// and the sums of all slots stay on the SM.  Large trees order a level's
+// parents by which of their 27 neighbours are split, so that a tile's targets
+// have the same slots.
+//
+// Per slot, with expansions of the level scaled by the box size w
+// (M~_n = w^-n M_n, L_j = w^-(j+1) L~_j; the factor w^-n rides on the phases):
+//   R  X = e^{i m phi} M~ (formed as operands are read), W_n = (P_n Re X_n,
+//      Q_n Im X_n) for orders n < p; and D += the whole map of the order-p
+//      moments into the potential local's frame of this azimuth
+//   T  Lz^k = T_k W^k, the distance in the operator
+//   I  S_j += (PB_j Re Lz_j, QB_j Im Lz_j), orders j <= p + 1
+// The potential local (order p, sources <= p) and the field local (order
+// p + 1, sources < p) differ by the order-p sources alone, so S serves both
+// and D is the rest.  S and D accumulate in registers over the slots of one
+// azimuth (36 of up to 189) and are then turned by e^{-i m phi} into the tile's
+// sums in shared memory, each element by its one owner: no atomics, and a
+// target's result does not depend on its tile (absent sources add zeros).
+//
+// A slot's operators (one class, 51 KB at p = 10) and the next slot's moments
+// come by bulk copies while the stages run; the moments, W and Lz change places
+// in two buffers.  Three barriers per slot of 32 columns.  Operand buffers are
+// laid out so that fragment loads and stores are free of bank conflicts.
+//
+// Before (one block per sibling group, 8-column tiles of one class, an operator
+// fragment load per MMA, five barriers per 8 columns), 4M Plummer points,
+// p = 10: 69.6 ms, the FP64 tensor pipe 24% busy.
+#include <cub/device/device_radix_sort.cuh>
+
+#include <algorithm>
+#include <vector>
+
+#include "m2l_tile.cuh"
+
+namespace sfmm {
+namespace {
+
+using tile::imin;
+using tile::up;
+
+struct OpsArgs {
+    const double* rot;
+    const int* rot_off;
+    int rot_len;
+    const double* tzx;
+    const int* tzx_off;
+};
+
+// Element (row, col) of fragment f of one class, P a run-time order (the
+// layout of tile::Frags<P>).
+__device__ double tile_entry(const OpsArgs& o, int P, int c, int f, int row, int col)
+{
+    const double* R = o.rot + int64_t(c) * o.rot_len;
+    const double rho = sqrt(double(tile::class_dist2(c)));
+    auto mat = [&](int n, int m, int r, int k) { return R[o.rot_off[n] + m * (n + 1) * (n + 1) + r * (n + 1) + k]; };
+    // z-translation between scaled expansions: target order j, source order n, azimuth k
+    auto tz = [&](int k, int j, int n) { return o.tzx[o.tzx_off[k] + (j - k) * (P + 1 - k) + (n - k)] * pow(rho, -double(j + n + 1)); };
+    // rotation of orders n < P: per (row tile, K chunk) P then Q
+    for (int n = 0; n < P; ++n) {
+        const int KC = up(n + 1, 4), cnt = 2 * up(n + 1, 8) * KC;
+        if (f < cnt) {
+            const int r = 8 * (f / 2 / KC) + row, k = 4 * (f / 2 % KC) + col;
+            if (r > n || k > n || ((f & 1) && (r == 0 || k == 0))) return 0.0;
+            return mat(n, f & 1, r, k);
+        }
+        f -= cnt;
+    }
+    for (int k = 0; k < P; ++k) {
+        const int KC = up(P - k, 4), cnt = up(P + 2 - k, 8) * KC;
+        if (f < cnt) {
+            const int j = k + 8 * (f / KC) + row, n = k + 4 * (f % KC) + col;
+            return j <= P + 1 && n <= P - 1 ? tz(k, j, n) : 0.0;
+        }
+        f -= cnt;
+    }
+    for (int j = 0; j <= P + 1; ++j) {
+        const int km = imin(j, P - 1), KP = up(km + 1, 4), KQ = up(km, 4), per = KP + KQ, cnt = up(j + 1, 8) * per;
+        if (f < cnt) {
+            const int r = 8 * (f / per) + row, h = f % per;
+            const int q = h >= KP, k = q ? 1 + 4 * (h - KP) + col : 4 * h + col;
+            if (r > j || k > km || (q && r == 0)) return 0.0;
+            return mat(j, 2 + q, r, k);
+        }
+        f -= cnt;
+    }
+    // D: potential local row (j, m) from the order-P moments k
+    const int T = (P + 1) * (P + 2) / 2, DK = up(P + 1, 4), dcnt = 2 * up(T, 8) * DK;
+    if (f < dcnt) {
+        const int r = 8 * (f / 2 / DK) + row, k = 4 * (f / 2 % DK) + col, q = f & 1;
+        if (r >= T || k > P || (q && k == 0)) return 0.0;
+        int j, m;
+        tri_nm(r, j, m);
+        if (q && m == 0) return 0.0;
+        double v = 0.0;
+        for (int b = q; b <= j; ++b) v += mat(j, 2 + q, m, b) * tz(b, j, P) * mat(P, q, b, k);
+        return v;
+    }
+    return 0.0;
+}
+
+__global__ void k_tile_ops(OpsArgs o, int P, int per_class, double* __restrict__ out)
+{
+    const int64_t total = int64_t(tile::kClasses) * per_class * 32;
+    for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < total; e += int64_t(gridDim.x) * blockDim.x) {
+        const int lane = static_cast<int>(e & 31), f = static_cast<int>((e >> 5) % per_class), c = static_cast<int>((e >> 5) / per_class);
+        // class 7 t2i + dk + 3; (0, 0, dk) with |dk| <= 1 and other adjacent offsets never occur as sources
+        out[e] = tile::class_dist2(c) > 0 ? tile_entry(o, P, c, f, lane >> 2, lane & 3) : 0.0;
+    }
+}
+
+int frags_per_class(int P)
+{
+    int s = 0;
+    for (int n = 0; n < P; ++n) s += 2 * up(n + 1, 8) * up(n + 1, 4);
+    s += 2 * up((P + 1) * (P + 2) / 2, 8) * up(P + 1, 4);
+    for (int k = 0; k < P; ++k) s += up(P + 2 - k, 8) * up(P - k, 4);
+    for (int j = 0; j <= P + 1; ++j) s += up(j + 1, 8) * (up(imin(j, P - 1) + 1, 4) + up(imin(j, P - 1), 4));
+    return s;
+}
+
+// Sort key of a split parent: its level, then which of its 27 neighbours are
+// split (they hold its children's sources).
+__global__ void k_tile_keys(const int32_t* __restrict__ list, int64_t n, const int64_t* __restrict__ lvl_off, int depth,
+                            const int32_t* __restrict__ colleague, const int32_t* __restrict__ nchild, uint32_t* __restrict__ key)
+{
+    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
+        const int g = list[i];
+        int l = 1;
+        while (l < depth && g >= lvl_off[l + 1]) ++l;
+        uint32_t m = 0;
+        for (int s = 0; s < 27; ++s) {
+            const int c = colleague[27 * int64_t(g) + s];
+            if (c >= 0 && nchild[c] > 0) m |= 1u << s;
+        }
+        key[i] = uint32_t(l) << 27 | m;
+    }
+}
+
+// Split tiles: the parts' sums added in part order, a warp per target.
+__global__ void k_tile_sum(EvalArgs a, tile::TileArgs g, int64_t chunks)
+{
+    const int lane = threadIdx.x & 31, qd = a.qdim;
+    const int64_t stride = (int64_t(gridDim.x) * blockDim.x) >> 5, total = chunks * 8 * g.tpb;
+    // the part sums of len coefficients from `first` on, then (more) the order-P sources'
+    auto sum = [&](const cplx* part, const cplx* more, int64_t first, int64_t len, cplx* out) {
+        for (int64_t e = lane; e < len; e += 32) {
+            cplx v = part[first + e];
+#pragma unroll
+            for (int q = 1; q < 2 * tile::kParts; ++q) {
+                if (q >= tile::kParts && !more) break;
+                const cplx w = (q < tile::kParts ? part : more)[(q % tile::kParts) * g.rows * (len / qd) + first + e];
+                v.re += w.re;
+                v.im += w.im;
+            }
+            out[e] = v;
+        }
+    };
+    for (int64_t w = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5; w < total; w += stride) {
+        const int64_t cell = w / g.tpb;
+        const int t = static_cast<int>(w % g.tpb), oct = static_cast<int>(cell & 7);
+        const int4 ck = g.chunk[cell >> 3];
+        if (t >= ck.y) continue;
+        const int pr = g.parent[ck.x + t], cb = a.child_beg[pr], nc = a.nchild[pr];
+        int64_t node = -1;
+        for (int k = 0; k < nc; ++k)
+            if (static_cast<int>(a.key[cb + k] & 7) == oct) node = cb + k;
+        if (node < 0) continue;
+        if (a.want_pot) sum(g.part_a, g.part_d, (node - g.node0) * qd * a.T, int64_t(qd) * a.T, a.LA + node * qd * a.T);
+        if (a.want_field) sum(g.part_b, nullptr, (node - g.node0) * qd * a.T1, int64_t(qd) * a.T1, a.LB + node * qd * a.T1);
+    }
+}
+
+}  // namespace
+
+void build_tile_ops(PlanTables& tb, int P, cudaStream_t st)
+{
+    const int nf = frags_per_class(P);
+    tb.tile_ops.alloc(size_t(tile::kClasses) * nf * 32, st);
+    tb.tile_zero.alloc(size_t(P + 1) * (P + 2), st);
+    SFMM_CUDA(cudaMemsetAsync(tb.tile_zero.ptr, 0, tb.tile_zero.bytes(), st));
+    OpsArgs o{tb.rot.ptr, tb.rot_off.ptr, tb.rot_len, tb.tzx.ptr, tb.tzx_off.ptr};
+    k_tile_ops<<<512, 256, 0, st>>>(o, P, nf, tb.tile_ops.ptr);
+    SFMM_CHECK_LAUNCH();
+}
+
+// Plans that run it: FP64 plans, and mixed plans whose M2L falls back to FP64
+// (a shard, the rotation switch) below the order the TF32 kernel takes.
+bool m2l_tile_supported(const Plan& pl)
+{
+    return pl.p >= kTileMinOrder && pl.p <= kTileMaxOrder && pl.tree->depth >= 2 && !pl.m2l_force_rows && !pl.i8 &&
+           !(pl.precision == FMM_PRECISION_MIXED && pl.p >= kTf32MinOrder);
+}
+
+// Tiles of the plan's tree (or of its shard's parents).  pl.sh_list / pl.sh_S
+// hold the split parents level by level.
+void m2l_tile_setup(Plan& pl)
+{
+    pl.mt_chunks = 0;
+    pl.mt_groups = 0;
+    pl.mt_on = false;
+    if (!m2l_tile_supported(pl)) return;
+    Tree& t = *pl.tree;
+    // sparse lists take the group kernel; a forest decides member by member, so that a member's result does not
+    // depend on its company
+    const bool forest = !t.member_sparse.empty();
+    bool some = forest ? false : m2l_sparse(t.il_nnz, t.n_nodes - t.lvl_off[2]), all = some;
+    if (forest) {
+        all = true;
+        for (uint8_t v : t.member_sparse) {
+            some |= v != 0;
+            all &= v != 0;
+        }
+    }
+    if (all) return;
+    pl.mt_on = true;
+    cudaStream_t st = t.ctx->stream;
+    const int sms = t.ctx->sm_count;
+    const int64_t n = pl.sh_S[t.depth];
+    if (n == 0) return;
+    // few targets: the parts of a tile in blocks of their own, and if that does not fill the SMs either, narrow tiles
+    const int64_t rows = (t.lvl_off[t.depth + 1] - t.lvl_off[2]) * pl.qdim;
+    const int full = tile::full_warps(pl.p);
+    pl.mt_split = rows < kTileSplitRows;
+    pl.mt_warps = pl.mt_split && rows * tile::kParts < int64_t(sms) * 4 * 8 * full ? tile::kSmallWarps : full;
+    pl.mt_tpb = 8 * pl.mt_warps / pl.qdim;
+    std::vector<int32_t> b(pl.sh_S), e(pl.sh_S);             // per level: parents [b, e)
+    for (int q = 1; q < t.depth; ++q) e[q] = pl.sh_S[q + 1];
+    pl.mt_parent.alloc(n, st);
+    const bool shard = pl.shard_count > 1;
+    if (some) {
+        // the forest's split parents, those of sparse members apart
+        std::vector<int32_t> list(n), tiled, group;
+        SFMM_CUDA(cudaMemcpyAsync(list.data(), pl.sh_list.ptr, n * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+        SFMM_CUDA(cudaStreamSynchronize(st));
+        const size_t B = t.member_sparse.size();
+        for (int q = 1; q < t.depth; ++q) {
+            const auto first = t.member_node.begin() + q * (B + 1);
+            b[q] = static_cast<int32_t>(tiled.size());
+            for (int32_t i = pl.sh_S[q]; i < pl.sh_S[q + 1]; ++i) {
+                const size_t r = std::upper_bound(first, first + B + 1, int64_t(list[i])) - first - 1;
+                (t.member_sparse[r] ? group : tiled).push_back(list[i]);
+            }
+            e[q] = static_cast<int32_t>(tiled.size());
+        }
+        pl.mt_groups = static_cast<int64_t>(group.size());
+        pl.mt_group.alloc(std::max<size_t>(group.size(), 1), st);
+        if (!group.empty())
+            SFMM_CUDA(cudaMemcpyAsync(pl.mt_group.ptr, group.data(), group.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st));
+        if (!tiled.empty())
+            SFMM_CUDA(cudaMemcpyAsync(pl.mt_parent.ptr, tiled.data(), tiled.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st));
+        SFMM_CUDA(cudaStreamSynchronize(st));
+    } else if (shard) {
+        std::vector<int32_t> list(n);
+        SFMM_CUDA(cudaMemcpyAsync(list.data(), pl.sh_list.ptr, n * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+        SFMM_CUDA(cudaStreamSynchronize(st));
+        for (int q = 1; q < t.depth; ++q) {
+            const auto lo = list.begin() + pl.sh_S[q], hi = list.begin() + pl.sh_S[q + 1];
+            b[q] = static_cast<int32_t>(std::lower_bound(lo, hi, pl.own_parent_b[q]) - list.begin());
+            e[q] = static_cast<int32_t>(std::lower_bound(lo, hi, pl.own_parent_e[q]) - list.begin());
+        }
+    }
+    if (!some && !shard && n >= kTileSortMin) {
+        DevBuf<uint32_t> k0, k1;
+        DevBuf<int64_t> lvl;
+        k0.alloc(n, st);
+        k1.alloc(n, st);
+        lvl.alloc(t.lvl_off.size(), st);
+        SFMM_CUDA(cudaMemcpyAsync(lvl.ptr, t.lvl_off.data(), t.lvl_off.size() * sizeof(int64_t), cudaMemcpyHostToDevice, st));
+        k_tile_keys<<<blocks_for(n, 256, int64_t(sms) * 8), 256, 0, st>>>(pl.sh_list.ptr, n, lvl.ptr, t.depth, t.colleague.ptr,
+                                                                         t.nchild.ptr, k0.ptr);
+        SFMM_CHECK_LAUNCH();
+        size_t tmp_bytes = 0;
+        SFMM_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, k0.ptr, k1.ptr, pl.sh_list.ptr, pl.mt_parent.ptr,
+                                                  static_cast<int>(n), 0, 32, st));
+        DevBuf<uint8_t> tmp;
+        tmp.alloc(std::max<size_t>(tmp_bytes, 1), st);
+        SFMM_CUDA(cub::DeviceRadixSort::SortPairs(tmp.ptr, tmp_bytes, k0.ptr, k1.ptr, pl.sh_list.ptr, pl.mt_parent.ptr,
+                                                  static_cast<int>(n), 0, 32, st));
+    } else if (!some) {
+        SFMM_CUDA(cudaMemcpyAsync(pl.mt_parent.ptr, pl.sh_list.ptr, n * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
+    }
+    std::vector<int4> ck;
+    for (int q = 1; q < t.depth; ++q)
+        for (int32_t s = b[q]; s < e[q]; s += pl.mt_tpb) ck.push_back(make_int4(s, imin(pl.mt_tpb, e[q] - s), q + 1, 0));
+    pl.mt_chunks = static_cast<int64_t>(ck.size());
+    if (ck.empty()) return;
+    pl.mt_chunk.alloc(ck.size(), st);
+    SFMM_CUDA(cudaMemcpyAsync(pl.mt_chunk.ptr, ck.data(), ck.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
+    const int64_t items = pl.mt_chunks * 8 * (pl.mt_split ? tile::kParts : 1);
+    const int64_t blocks = std::min<int64_t>(items, int64_t(sms) * tile::max_per_sm(pl.mt_warps));
+    pl.mt_table.alloc(size_t(blocks) * 2 * tile::kSlots * 8 * pl.mt_warps, st);
+    pl.mt_part.release();
+    if (pl.mt_split) pl.mt_part.alloc(size_t(tile::kParts) * rows * (2 * pl.T + pl.T1), st);
+}
+
+bool launch_m2l_tile(Plan& pl, const EvalArgs& a, cudaStream_t st)
+{
+    if (!pl.mt_on || !m2l_tile_supported(pl)) return false;
+    const Tree& t = *pl.tree;
+    const int sms = t.ctx->sm_count;
+    if (pl.mt_groups > 0) {
+        EvalArgs b = a;
+        b.m2l_list = pl.mt_group.ptr;
+        launch_m2l(b, 0, pl.mt_groups, sms, st);
+    }
+    if (pl.mt_chunks == 0) return true;                      // no (other) targets
+    tile::TileArgs g{};
+    g.ops = pl.tab->tile_ops.ptr;
+    g.parent = pl.mt_parent.ptr;
+    g.chunk = pl.mt_chunk.ptr;
+    g.items = pl.mt_chunks * 8 * (pl.mt_split ? tile::kParts : 1);
+    g.tpb = pl.mt_tpb;
+    g.split = pl.mt_split;
+    g.node0 = t.lvl_off[2];
+    g.rows = (t.lvl_off[t.depth + 1] - t.lvl_off[2]) * pl.qdim;
+    g.part_a = reinterpret_cast<cplx*>(pl.mt_part.ptr);
+    g.part_d = g.part_a + tile::kParts * g.rows * pl.T;
+    g.part_b = g.part_d + tile::kParts * g.rows * pl.T;
+    g.table = pl.mt_table.ptr;
+    g.zero = reinterpret_cast<const cplx*>(pl.tab->tile_zero.ptr);
+    g.ctr = pl.m2l_ctr.ptr;
+    const bool done = a.p <= 6   ? tile::launch_lo(a, g, pl.mt_warps, sms, st)
+                      : a.p <= 9 ? tile::launch_mid(a, g, pl.mt_warps, sms, st)
+                                 : tile::launch_hi(a, g, pl.mt_warps, sms, st);
+    if (done && pl.mt_split) {
+        k_tile_sum<<<blocks_for(pl.mt_chunks * 8 * pl.mt_tpb * 32, 256, int64_t(sms) * 16), 256, 0, st>>>(a, g, pl.mt_chunks);
+        SFMM_CHECK_LAUNCH();
+    }
+    return done;
+}
+
+}  // namespace sfmm

@@ -99,6 +99,8 @@ size_t estimate_bytes(int64_t n, int p, int qdim, int leaf, int precision)
     // are first allocated for n / 8 nodes (15 B per point)
     const double per_point = 48 + 48 + 48 + 8.0 * (qdim + 3) * 3 + 16;
     double per_node = 16.0 * qdim * (2 * T + T1) + 190 * 8 + 64;         // M, LA, LB, ilist, node arrays
+    // the tiled FP64 M2L of small trees: the parts' sums
+    if (precision == FMM_PRECISION_FP64 && nodes * qdim < 24 * 1024) per_node += 6 * 16.0 * qdim * (2 * T + T1);
     // mixed plans' tensor-core M2L (m2l_i8.cu): slot table, block lists and
     // four digits of the padded real moments per node
     if (precision == FMM_PRECISION_MIXED && p <= sfmm::kI8MaxOrder)

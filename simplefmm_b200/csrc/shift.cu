@@ -97,14 +97,14 @@ __global__ void k_has_children(const int32_t* __restrict__ nchild, int64_t base,
         flag[i] = nchild[base + i] > 0 ? 1 : 0;
 }
 
-// slot -> node, and the slot of each level's first parent (S[q], q = 2..depth; S[depth] = total)
+// slot -> node, and the slot of each level's first parent (S[q], q = 1..depth; S[depth] = total)
 __global__ void k_slots(const int32_t* __restrict__ flag, const int32_t* __restrict__ slot, int64_t base, int64_t n,
                         int32_t* __restrict__ list, const int64_t* __restrict__ lvl, int depth, int32_t* __restrict__ S)
 {
     for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
         if (flag[i]) list[slot[i]] = static_cast<int32_t>(base + i);
     if (blockIdx.x == 0 && threadIdx.x == 0)
-        for (int q = 2; q <= depth; ++q) {
+        for (int q = 1; q <= depth; ++q) {
             const int64_t i = lvl[q] - base;
             S[q] = i < n ? slot[i] : (n ? slot[n - 1] + flag[n - 1] : 0);
         }
@@ -383,12 +383,12 @@ void shift_setup(Plan& pl)
 {
     Tree& t = *pl.tree;
     pl.shift_on = false;
-    if (t.depth < 3) return;
+    if (t.depth < 2) return;
     Context& c = *t.ctx;
     cudaStream_t st = c.stream;
     const int RA = 2 * pl.T, RB = 2 * pl.T1;
-    // parents of levels 2 .. depth - 1 with children: compact slots
-    const int64_t base = t.lvl_off[2], n = t.lvl_off[t.depth] - base;
+    // parents of levels 1 .. depth - 1 with children: compact slots
+    const int64_t base = t.lvl_off[1], n = t.lvl_off[t.depth] - base;
     DevBuf<int32_t> flag;
     flag.alloc(n, st);
     pl.sh_slot.alloc(n + 1, st);                        // exclusive scans write n + 1 entries
@@ -406,6 +406,7 @@ void shift_setup(Plan& pl)
     pl.sh_S.assign(t.depth + 1, 0);
     SFMM_CUDA(cudaMemcpyAsync(pl.sh_S.data(), S.ptr, (t.depth + 1) * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     SFMM_CUDA(cudaStreamSynchronize(st));
+    if (t.depth < 3) return;
     // maps per children level 3 .. depth, fragment order: OpM (RA x 8RA),
     // OpLA (8RA x RA), OpLB (8RB x RB); zero padding rows / columns; each
     // the order's maps at rho = 1 scaled to the level's rho
