@@ -228,11 +228,13 @@ void m2l_tile_setup(Plan& pl)
     const int sms = t.ctx->sm_count;
     const int64_t n = pl.sh_S[t.depth];
     if (n == 0) return;
-    // few targets: the parts of a tile in blocks of their own, and if that does not fill the SMs either, narrow tiles
+    // few targets: the parts of a tile in blocks of their own, and if that does not give every SM two full blocks to
+    // run one after the other, narrow tiles (p = 10 at one, two and four blocks, M2L: Plummer 100k points 1.35, 1.35
+    // and 1.92 ms; p = 6, 60k 0.57, 0.46 and 0.46 ms)
     const int64_t rows = (t.lvl_off[t.depth + 1] - t.lvl_off[2]) * pl.qdim;
     const int full = tile::full_warps(pl.p);
     pl.mt_split = rows < kTileSplitRows;
-    pl.mt_warps = pl.mt_split && rows * tile::kParts < int64_t(sms) * 4 * 8 * full ? tile::kSmallWarps : full;
+    pl.mt_warps = pl.mt_split && rows * tile::kParts < int64_t(sms) * 2 * 8 * full ? tile::kSmallWarps : full;
     pl.mt_tpb = 8 * pl.mt_warps / pl.qdim;
     std::vector<int32_t> b(pl.sh_S), e(pl.sh_S);             // per level: parents [b, e)
     for (int q = 1; q < t.depth; ++q) e[q] = pl.sh_S[q + 1];
