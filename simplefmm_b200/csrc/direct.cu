@@ -1,8 +1,15 @@
 // Direct FP64 sums at selected targets -- the reference's accuracy check
-// (main.cpp:70-111) on the device: thread per target, source tiles staged
-// in shared memory.  Used to state the FMM error against the exact sum.
+// (main.cpp:70-111) on the device: two targets per thread, source records
+// staged in shared memory and read by broadcast.  Used to state the FMM error
+// against the exact sum.
+//
+// Bound: the FP64 pipe, about 20 instructions a pair with 1/r from rsqrt and no
+// division: 10,000 targets x 400,000 points 6.0 ms (the call 29.2 -> 6.5 ms);
+// 28.1 ms with a square root, a division by r and three by r^3 a pair and one
+// target per thread.
 #include "fmm_internal.cuh"
 
+#include <algorithm>
 #include <mutex>
 
 namespace sfmm {
@@ -12,56 +19,115 @@ std::atomic<long long> g_launches{0};
 namespace {
 
 constexpr int kThreads = 128;
+constexpr int kPerThread = 2;                             // targets per thread
+constexpr int kTargets = kThreads * kPerThread;           // targets per block
+constexpr int kTile = 128;                                // sources per tile
 
-__global__ void __launch_bounds__(kThreads) k_direct(const double* __restrict__ xyz, int64_t n,
-                                                     const double* __restrict__ Q, int qdim,
-                                                     const int64_t* __restrict__ targets, int64_t nt,
-                                                     int64_t chunk, double* __restrict__ part)
+// One staged tile against the thread's targets.  SELF: some target of the warp
+// is among the tile's sources; ks is its slot (the pair is left out).
+template<int QD, bool SELF>
+__device__ __forceinline__ void direct_tile(const double4* __restrict__ s4, const double2* __restrict__ s2, int cnt,
+                                            const double (&x)[kPerThread][3], const int64_t (&ks)[kPerThread],
+                                            double (&pa)[kPerThread][QD], double (&fa)[kPerThread][3])
 {
-    __shared__ double s[kThreads][6];
-    const int64_t t = blockIdx.x * int64_t(kThreads) + threadIdx.x;
-    const int64_t ti = t < nt ? targets[t] : -1;
-    // a target index outside [0, n) reads nothing; k_direct_sum reports it
-    const bool on = ti >= 0 && ti < n;
-    const int64_t i = on ? ti : 0;
-    const double xi = on ? xyz[3 * i] : 0, yi = on ? xyz[3 * i + 1] : 0, zi = on ? xyz[3 * i + 2] : 0;
-    double pa[3] = {0, 0, 0}, fa[3] = {0, 0, 0};
-    // sources [jb, je) of this block's chunk (blockIdx.y)
-    const int64_t jb = blockIdx.y * chunk;
-    const int64_t je = jb + chunk < n ? jb + chunk : n;
-    for (int64_t j0 = jb; j0 < je; j0 += kThreads) {
-        __syncthreads();
-        const int64_t j = j0 + threadIdx.x;
-        if (j < je) {
-            s[threadIdx.x][0] = xyz[3 * j];
-            s[threadIdx.x][1] = xyz[3 * j + 1];
-            s[threadIdx.x][2] = xyz[3 * j + 2];
-            for (int b = 0; b < qdim; ++b) s[threadIdx.x][3 + b] = Q[j * qdim + b];
-        }
-        __syncthreads();
-        const int cnt = je - j0 < kThreads ? static_cast<int>(je - j0) : kThreads;
-        if (!on) continue;
-        for (int k = 0; k < cnt; ++k) {
-            if (j0 + k == i) continue;
-            const double dx = xi - s[k][0], dy = yi - s[k][1], dz = zi - s[k][2];
-            const double r = sqrt(dx * dx + dy * dy + dz * dz);
-            const double r3 = r * r * r;
-            for (int b = 0; b < qdim; ++b) pa[b] += s[k][3 + b] / r;
-            if (qdim == 1) {
-                fa[0] += s[k][3] * dx / r3;
-                fa[1] += s[k][3] * dy / r3;
-                fa[2] += s[k][3] * dz / r3;
-            } else if (qdim == 3) {
-                fa[0] += (s[k][4] * dz - s[k][5] * dy) / r3;
-                fa[1] += (s[k][5] * dx - s[k][3] * dz) / r3;
-                fa[2] += (s[k][3] * dy - s[k][4] * dx) / r3;
+#pragma unroll 2
+    for (int k = 0; k < cnt; ++k) {
+        const double4 v = s4[k];
+        const double2 w = QD > 1 ? s2[k] : make_double2(0, 0);
+#pragma unroll
+        for (int u = 0; u < kPerThread; ++u) {
+            if (SELF && k == ks[u]) continue;
+            const double dx = x[u][0] - v.x, dy = x[u][1] - v.y, dz = x[u][2] - v.z;
+            const double ir = rsqrt(fma(dx, dx, fma(dy, dy, dz * dz)));
+            const double ir3 = ir * ir * ir;
+            pa[u][0] = fma(v.w, ir, pa[u][0]);
+            if (QD > 1) pa[u][1] = fma(w.x, ir, pa[u][1]);
+            if (QD > 2) pa[u][2] = fma(w.y, ir, pa[u][2]);
+            if (QD == 1) {
+                const double c = v.w * ir3;
+                fa[u][0] = fma(c, dx, fa[u][0]);
+                fa[u][1] = fma(c, dy, fa[u][1]);
+                fa[u][2] = fma(c, dz, fa[u][2]);
+            } else if (QD == 3) {
+                fa[u][0] = fma(w.x * dz - w.y * dy, ir3, fa[u][0]);
+                fa[u][1] = fma(w.y * dx - v.w * dz, ir3, fa[u][1]);
+                fa[u][2] = fma(v.w * dy - w.x * dx, ir3, fa[u][2]);
             }
         }
     }
-    if (!on) return;
-    double* o = part + (blockIdx.y * nt + t) * 6;
-    for (int b = 0; b < 3; ++b) o[b] = pa[b];
-    for (int c = 0; c < 3; ++c) o[3 + c] = fa[c];
+}
+
+template<int QD>
+__global__ void __launch_bounds__(kThreads) k_direct(const double* __restrict__ xyz, int64_t n, const double* __restrict__ Q,
+                                                     const int64_t* __restrict__ targets, int64_t nt, int64_t chunk,
+                                                     double* __restrict__ part)
+{
+    __shared__ double4 s4[kTile];
+    __shared__ double2 s2[QD > 1 ? kTile : 1];
+    int64_t t[kPerThread], i[kPerThread];
+    bool on[kPerThread];
+    double x[kPerThread][3], pa[kPerThread][QD] = {}, fa[kPerThread][3] = {};
+#pragma unroll
+    for (int u = 0; u < kPerThread; ++u) {
+        t[u] = blockIdx.x * int64_t(kTargets) + u * kThreads + threadIdx.x;
+        const int64_t ti = t[u] < nt ? targets[t[u]] : -1;
+        // a target index outside [0, n) reads nothing; k_direct_sum reports it
+        on[u] = ti >= 0 && ti < n;
+        i[u] = on[u] ? ti : -1;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) x[u][c] = on[u] ? xyz[3 * i[u] + c] : 0.0;
+    }
+    // sources [jb, je) of this block's chunk (blockIdx.y)
+    const int64_t jb = blockIdx.y * chunk;
+    const int64_t je = jb + chunk < n ? jb + chunk : n;
+    for (int64_t j0 = jb; j0 < je; j0 += kTile) {
+        const int cnt = je - j0 < kTile ? static_cast<int>(je - j0) : kTile;
+        __syncthreads();
+        for (int k = threadIdx.x; k < cnt; k += kThreads) {
+            const int64_t j = j0 + k;
+            s4[k] = make_double4(xyz[3 * j], xyz[3 * j + 1], xyz[3 * j + 2], Q[j * QD]);
+            if (QD > 1) s2[k] = make_double2(Q[j * QD + 1], QD > 2 ? Q[j * QD + QD - 1] : 0.0);
+        }
+        __syncthreads();
+        int64_t ks[kPerThread];
+        bool self = false;
+#pragma unroll
+        for (int u = 0; u < kPerThread; ++u) {
+            ks[u] = i[u] - j0;
+            self |= ks[u] >= 0 && ks[u] < cnt;
+        }
+        if (__any_sync(0xffffffffu, self))
+            direct_tile<QD, true>(s4, s2, cnt, x, ks, pa, fa);
+        else
+            direct_tile<QD, false>(s4, s2, cnt, x, ks, pa, fa);
+    }
+#pragma unroll
+    for (int u = 0; u < kPerThread; ++u) {
+        if (!on[u]) continue;
+        double* o = part + (blockIdx.y * nt + t[u]) * 6;
+        for (int b = 0; b < 3; ++b) o[b] = b < QD ? pa[u][b < QD ? b : 0] : 0.0;
+        for (int c = 0; c < 3; ++c) o[3 + c] = fa[u][c];
+    }
+}
+
+// Source chunks: enough blocks to fill the device several times over, at least
+// 512 sources each, at most `most` chunks.
+int64_t direct_chunks(int64_t n, int64_t nt, int sms, int64_t most)
+{
+    const int64_t gx = (nt + kTargets - 1) / kTargets;
+    const int64_t want = std::max<int64_t>(1, (int64_t(sms) * 16 + gx - 1) / gx);
+    return std::max<int64_t>(1, std::min(std::min(want, std::max<int64_t>(1, n / 512)), std::min<int64_t>(most, 65535)));
+}
+
+void launch_direct(const double* xyz, int64_t n, const double* Q, int qdim, const int64_t* targets, int64_t nt, int64_t nchunk,
+                   double* part, cudaStream_t st)
+{
+    const int64_t chunk = (n + nchunk - 1) / nchunk;
+    const dim3 grid(static_cast<unsigned>((nt + kTargets - 1) / kTargets), static_cast<unsigned>(nchunk));
+    if (qdim == 1) k_direct<1><<<grid, kThreads, 0, st>>>(xyz, n, Q, targets, nt, chunk, part);
+    else if (qdim == 2) k_direct<2><<<grid, kThreads, 0, st>>>(xyz, n, Q, targets, nt, chunk, part);
+    else k_direct<3><<<grid, kThreads, 0, st>>>(xyz, n, Q, targets, nt, chunk, part);
+    SFMM_CHECK_LAUNCH();
 }
 
 // Sum the chunks' partial sums in chunk order (deterministic).  A target
@@ -97,17 +163,10 @@ void direct_sum(Context& c, const double* xyz, int64_t n, const double* Q, int q
                 double* pot, double* field, int* bad)
 {
     if (nt <= 0) return;
-    // split the sources into chunks so that small target sets still fill the device
-    const int64_t gx = (nt + kThreads - 1) / kThreads;
-    int64_t nchunk = std::max<int64_t>(1, (int64_t(c.sm_count) * 8 + gx - 1) / gx);
-    nchunk = std::min<int64_t>(nchunk, std::max<int64_t>(1, n / (4 * kThreads)));
-    nchunk = std::min<int64_t>(nchunk, 65535);
-    const int64_t chunk = (n + nchunk - 1) / nchunk;
+    const int64_t nchunk = direct_chunks(n, nt, c.sm_count, 65535);
     DevBuf<double> part;
     part.alloc(size_t(nchunk) * nt * 6, c.stream);
-    k_direct<<<dim3(static_cast<unsigned>(gx), static_cast<unsigned>(nchunk)), kThreads, 0, c.stream>>>(
-        xyz, n, Q, qdim, targets, nt, chunk, part.ptr);
-    SFMM_CHECK_LAUNCH();
+    launch_direct(xyz, n, Q, qdim, targets, nt, nchunk, part.ptr, c.stream);
     k_direct_sum<<<static_cast<unsigned>((nt + 255) / 256), 256, 0, c.stream>>>(
         part.ptr, nt, static_cast<int>(nchunk), qdim, targets, n, pot, field, bad);
     SFMM_CHECK_LAUNCH();
@@ -177,17 +236,10 @@ extern "C" int fmm_direct_noalloc(const double* xyz, int64_t n, const double* Q,
         const NoAllocDevice d = noalloc_device(dev);
         cudaStream_t st = static_cast<cudaStream_t>(stream);
         // chunking as direct_sum, capped by the scratch size
-        const int64_t gx = (nt + kThreads - 1) / kThreads;
-        int64_t nchunk = std::max<int64_t>(1, (int64_t(d.sms) * 8 + gx - 1) / gx);
-        nchunk = std::min<int64_t>(nchunk, std::max<int64_t>(1, n / (4 * kThreads)));
-        nchunk = std::min<int64_t>(nchunk, kNoAllocScratchDoubles / (6 * nt));
-        nchunk = std::min<int64_t>(nchunk, 65535);
-        const int64_t chunk = (n + nchunk - 1) / nchunk;
+        const int64_t nchunk = direct_chunks(n, nt, d.sms, kNoAllocScratchDoubles / (6 * nt));
         // every (chunk, target) slot of the scratch is written before it is
         // read, so nothing left by an earlier call needs clearing
-        k_direct<<<dim3(static_cast<unsigned>(gx), static_cast<unsigned>(nchunk)), kThreads, 0, st>>>(
-            xyz, n, Q, qdim, targets, nt, chunk, d.scratch);
-        SFMM_CHECK_LAUNCH();
+        launch_direct(xyz, n, Q, qdim, targets, nt, nchunk, d.scratch, st);
         // a target index outside [0, n) is not read: its outputs become NaN
         k_direct_sum<<<static_cast<unsigned>((nt + 255) / 256), 256, 0, st>>>(
             d.scratch, nt, static_cast<int>(nchunk), qdim, targets, n, pot, field, nullptr);
