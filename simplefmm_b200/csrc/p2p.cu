@@ -15,6 +15,8 @@
 // its targets; every source read from shared memory is applied to the lane's
 // target of every pass (register blocking over passes).  Slices of a target
 // are summed with xor shuffles at the end.
+#include <type_traits>
+
 #include "eval_util.cuh"
 
 namespace sfmm {
@@ -506,6 +508,130 @@ __device__ __forceinline__ void p2p_mixed_tile(const float4* __restrict__ sxq, c
 }
 
 
+// Packed FP32 pairs (two IEEE operations per instruction, each rounded as the
+// scalar one).
+__device__ __forceinline__ uint64_t pk(float a, float b)
+{
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unpk(uint64_t v)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
+{
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ float rsqrt_approx(float r2)
+{
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(r2));
+    return y;
+}
+
+// Scalar charges: the tile's sources k and k + slices of a lane side by side,
+// so that one packed instruction does the same step of both; the sums still
+// take them in order.  Coordinates are stored negated (a - b = a + (-b)).  The
+// same operations and roundings as p2p_mixed_tile, 31 instead of 54
+// instructions for two pairs: the loop is bound by instruction issue.
+struct PairTile {
+    ulonglong2 *a, *b, *c;                // (x x', y y'), (z z', q q') high parts and charges; (x x', y y') low parts
+    uint64_t* d;                          // (z z') low parts
+};
+constexpr int kPairs = kChunk / 2;
+
+__device__ __forceinline__ void pair_store(const PairTile& t, int k, int log_s, const F2& x, const F2& y, const F2& z, float q)
+{
+    const int s = 1 << log_s;
+    const int pair = (k >> (log_s + 1) << log_s) + (k & (s - 1)), h = k >> log_s & 1;
+    float *a = reinterpret_cast<float*>(t.a + pair) + h, *b = reinterpret_cast<float*>(t.b + pair) + h;
+    float *c = reinterpret_cast<float*>(t.c + pair) + h, *d = reinterpret_cast<float*>(t.d + pair) + h;
+    a[0] = -x.h;
+    a[2] = -y.h;
+    b[0] = -z.h;
+    b[2] = q;
+    c[0] = -x.l;
+    c[2] = -y.l;
+    d[0] = -z.l;
+}
+
+template<int NP, bool POT, bool FLD, bool SELF, int NO, int MP>
+__device__ __forceinline__ void p2p_mixed_pairs(const PairTile& tile, int s, int slices, int fill, const F2 (&xi)[MP], const F2 (&yi)[MP],
+                                                const F2 (&zi)[MP], const int (&ks)[MP], float (&part)[MP][NO > 0 ? NO : 1])
+{
+    uint64_t xh[NP], yh[NP], zh[NP], xl[NP], yl[NP], zl[NP];
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+        xh[p] = pk(xi[p].h, xi[p].h);
+        yh[p] = pk(yi[p].h, yi[p].h);
+        zh[p] = pk(zi[p].h, zi[p].h);
+        xl[p] = pk(xi[p].l, xi[p].l);
+        yl[p] = pk(yi[p].l, yi[p].l);
+        zl[p] = pk(zi[p].l, zi[p].l);
+    }
+    const uint64_t mhalf = pk(-0.5f, -0.5f), half = pk(0.5f, 0.5f);
+    int pair = s;
+    for (int k = s; k < fill; k += 2 * slices, pair += slices) {
+        const ulonglong2 ta = tile.a[pair], tb = tile.b[pair], tc = tile.c[pair];
+        const uint64_t td = tile.d[pair];
+        const bool two = k + slices < fill;               // the last pair of a lane may hold one source
+        const float2 q = unpk(tb.y);
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+            const uint64_t dx = add2(add2(xh[p], ta.x), add2(xl[p], tc.x));
+            const uint64_t dy = add2(add2(yh[p], ta.y), add2(yl[p], tc.y));
+            const uint64_t dz = add2(add2(zh[p], tb.x), add2(zl[p], td));
+            const uint64_t r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
+            // rsqrt_newton of both
+            const float2 r = unpk(r2);
+            const float y0 = rsqrt_approx(r.x), y1 = rsqrt_approx(r.y);
+            const uint64_t y = pk(y0, y1), yc = pk(fminf(y0, 8.507059e37f), fminf(y1, 8.507059e37f));
+            const uint64_t e = fma2(mul2(mul2(mhalf, r2), yc), yc, half);
+            uint64_t ir2 = fma2(y, e, y);
+            if (SELF) {
+                const float2 v = unpk(ir2);
+                ir2 = pk(k == ks[p] ? 0.f : v.x, k + slices == ks[p] ? 0.f : v.y);
+            }
+            const float2 ir = unpk(ir2);
+            if (POT) {
+                part[p][0] = fmaf(q.x, ir.x, part[p][0]);
+                if (two) part[p][0] = fmaf(q.y, ir.y, part[p][0]);
+            }
+            if (FLD) {
+                constexpr int o = POT ? 1 : 0;
+                const float2 cq = unpk(mul2(tb.y, mul2(mul2(ir2, ir2), ir2)));
+                const float2 fx = unpk(dx), fy = unpk(dy), fz = unpk(dz);
+                part[p][o] = fmaf(cq.x, fx.x, part[p][o]);
+                part[p][o + 1] = fmaf(cq.x, fy.x, part[p][o + 1]);
+                part[p][o + 2] = fmaf(cq.x, fz.x, part[p][o + 2]);
+                if (two) {
+                    part[p][o] = fmaf(cq.y, fx.y, part[p][o]);
+                    part[p][o + 1] = fmaf(cq.y, fy.y, part[p][o + 1]);
+                    part[p][o + 2] = fmaf(cq.y, fz.y, part[p][o + 2]);
+                }
+            }
+        }
+    }
+}
+
 template<int QD, bool POT, bool FLD, int kMaxPass, int MINB>
 __global__ void __launch_bounds__(kWarps * 32, MINB) k_p2p_mixed(EvalArgs a)
 {
@@ -517,6 +643,12 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_p2p_mixed(EvalArgs a)
     float4* sxq = reinterpret_cast<float4*>(mine);                 // x y z q0, high parts (leaf-centred)
     float4* sxl = sxq + kChunk;                                     // x y z low parts
     float2* sq12 = reinterpret_cast<float2*>(mine + kChunk * 32);   // only for QD > 1
+    // scalar charges: pairs of sources in the same space
+    PairTile pairs;
+    pairs.a = reinterpret_cast<ulonglong2*>(mine);
+    pairs.b = pairs.a + kPairs;
+    pairs.c = pairs.b + kPairs;
+    pairs.d = reinterpret_cast<uint64_t*>(pairs.c + kPairs);
     const double* q0 = a.qs;
     const double* q1 = a.qs + (QD > 1 ? a.n : 0);
     const double* q2 = a.qs + (QD > 2 ? 2 * a.n : 0);
@@ -538,6 +670,7 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_p2p_mixed(EvalArgs a)
             const int slices = 32 / tg;
             const int passes = (nt + tg - 1) / tg;
             const int ti = lane / slices, s = lane - ti * slices;
+            const int log_s = __ffs(slices) - 1;
             F2 xi[kMaxPass], yi[kMaxPass], zi[kMaxPass];
             int ii[kMaxPass];
             Sum2 acc[kMaxPass][NO > 0 ? NO : 1];
@@ -565,6 +698,10 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_p2p_mixed(EvalArgs a)
                     for (int k = lane; k < len; k += 32) {
                         const int j = j0 + k;
                         const F2 x = split_f(a.px[j] - c[0]), y = split_f(a.py[j] - c[1]), z = split_f(a.pz[j] - c[2]);
+                        if (QD == 1) {
+                            pair_store(pairs, fill + k, log_s, x, y, z, static_cast<float>(q0[j]));
+                            continue;
+                        }
                         sxq[fill + k] = make_float4(x.h, y.h, z.h, static_cast<float>(q0[j]));
                         sxl[fill + k] = make_float4(x.l, y.l, z.l, 0.f);
                         if (QD > 1) sq12[fill + k] = make_float2(static_cast<float>(q1[j]), static_cast<float>(q2[j]));
@@ -594,7 +731,20 @@ __global__ void __launch_bounds__(kWarps * 32, MINB) k_p2p_mixed(EvalArgs a)
                     ks[p] = ii[p] >= 0 && d < static_cast<unsigned>(self_len) ? self_s0 + static_cast<int>(d) : -1;
                 }
                 static_assert(kMaxPass <= 3, "passes dispatched up to 3");
-                if (passes == 1)
+                if constexpr (QD == 1) {
+                    // tiles that hold none of the leaf's own points (all but one of a leaf's, mostly) skip the self test
+                    auto run = [&](auto np, auto self) {
+                        p2p_mixed_pairs<decltype(np)::value, POT, FLD, decltype(self)::value, NO>(pairs, s, slices, fill, xi, yi, zi,
+                                                                                                  ks, part);
+                    };
+                    auto passed = [&](auto np) {
+                        if (self_len > 0) run(np, std::true_type{});
+                        else run(np, std::false_type{});
+                    };
+                    if (passes == 1) passed(std::integral_constant<int, 1>{});
+                    else if (passes == 2) passed(std::integral_constant<int, (kMaxPass >= 2 ? 2 : 1)>{});
+                    else passed(std::integral_constant<int, kMaxPass>{});
+                } else if (passes == 1)
                     p2p_mixed_tile<1, QD, POT, FLD, NO>(sxq, sxl, sq12, s, slices, fill, xi, yi, zi, ks, part);
                 else if (passes == 2)
                     p2p_mixed_tile<(kMaxPass >= 2 ? 2 : 1), QD, POT, FLD, NO>(sxq, sxl, sq12, s, slices, fill, xi, yi, zi, ks, part);
