@@ -175,7 +175,7 @@ struct Plan {
     // maps; compact slots of the parents that have children (levels >= 1)
     bool shift_on = false;
     DevBuf<double> sh_ops;
-    DevBuf<int32_t> sh_slot, sh_list;
+    DevBuf<int32_t> sh_slot, sh_list, sh_kid;
     std::vector<int32_t> sh_S;
     DevBuf<float2> m32;                       // mixed precision: scaled FP32 source moments
     // timing: evaluation start, far field (upward, M2L, downward) ends, end;

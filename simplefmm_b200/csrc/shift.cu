@@ -12,17 +12,20 @@
 //        stacked in octant order (absent children are zero);
 //   L2L  OpL (8R x R): rows oct * R + i, one product gives all eight
 //        children's shifts of a parent's local.
-// Only parents with children take part (compact slots from a scan at
-// set-up).  A block takes 32 (M2M) or 64 (L2L) columns (parent slot x charge
-// component); K chunks that hold only zero operator entries (the maps are
-// triangular in the expansion order) are skipped:
-//   k_m2m_mma  for each octant, stages the 32 children's moments in shared
-//              memory (the B operand) and accumulates OpM's octant block on the
-//              FP64 tensor cores (mma.sync m8n8k4, operator fragments read
-//              from L2 once per 4 column tiles); then writes the parents.
-//   k_l2l_mma  stages the 64 parents' locals, and for each 8-row tile of OpL
-//              adds the product into the child of that row's octant (each
-//              child coefficient has one writer: no atomics, deterministic).
+// Only parents with children take part (compact slots from a scan at set-up,
+// with each slot's child per octant).  K chunks that hold only zero operator
+// entries (the maps are triangular in the expansion order) are skipped:
+//   k_m2m_mma  16 columns (parent slot x charge component) and four 8-row tiles
+//              per block, a warp per octant: each sums its octant's products on
+//              the FP64 tensor cores (mma.sync m8n8k4, both operands read from
+//              L2), then the eight are added in octant order.  A level is a
+//              chain of at most 39 K chunks whatever its size; one warp taking
+//              the eight octants in turn (32 columns a block, the children
+//              staged per octant) took 90 us for a level of a few boxes.
+//   k_l2l_mma  stages the parents' locals, and for each 8-row tile of OpL adds
+//              the product into the child of that row's octant (each child
+//              coefficient has one writer: no atomics, deterministic); 64
+//              columns a block, 16 for levels that would leave SMs idle.
 // The sums differ from the direct ones in rounding order only (FP64, about
 // 1e-16 relative per term).  Evaluations allocate nothing here, so they can
 // be captured as CUDA graphs.
@@ -30,15 +33,17 @@
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 namespace sfmm {
 namespace {
 
-constexpr int kShiftCols = 32;            // M2M columns per block: four 8-column MMA tiles
+constexpr int kM2MTiles = 2;              // M2M: two 8-column MMA tiles per block
+constexpr int kM2MRows = 4;               // M2M: row tiles per block
 constexpr int kL2LTiles = 8;              // L2L: eight 8-column MMA tiles (64 columns) per block
+constexpr int kL2LSmallTiles = 2;         // small levels: two
 constexpr int kL2LRowGroups = 4;          // L2L: the 8R output rows split over at least 4 blocks
-constexpr int kM2MRowGroups = 2;          // M2M: the R output rows split over 2 blocks
 constexpr int kShiftWarps = 8;
 
 __host__ __device__ constexpr int cdiv(int a, int b) { return (a + b - 1) / b; }
@@ -98,11 +103,28 @@ __global__ void k_has_children(const int32_t* __restrict__ nchild, int64_t base,
 }
 
 // slot -> node, and the slot of each level's first parent (S[q], q = 1..depth; S[depth] = total)
+// and each slot's child per octant (-1 absent)
 __global__ void k_slots(const int32_t* __restrict__ flag, const int32_t* __restrict__ slot, int64_t base, int64_t n,
-                        int32_t* __restrict__ list, const int64_t* __restrict__ lvl, int depth, int32_t* __restrict__ S)
+                        const int32_t* __restrict__ child_beg, const int32_t* __restrict__ nchild, const uint64_t* __restrict__ key,
+                        int32_t* __restrict__ list, int32_t* __restrict__ kid, const int64_t* __restrict__ lvl, int depth,
+                        int32_t* __restrict__ S)
 {
     for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
-        if (flag[i]) list[slot[i]] = static_cast<int32_t>(base + i);
+        if (flag[i]) {
+            const int64_t s = slot[i];
+            list[s] = static_cast<int32_t>(base + i);
+            int32_t k8[8] = {-1, -1, -1, -1, -1, -1, -1, -1};
+            const int cb = child_beg[base + i], nc = nchild[base + i];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const int o = k < nc ? static_cast<int>(key[cb + k] & 7) : -1;
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if (u == o) k8[u] = cb + k;
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) kid[8 * s + u] = k8[u];
+        }
     if (blockIdx.x == 0 && threadIdx.x == 0)
         for (int q = 1; q <= depth; ++q) {
             const int64_t i = lvl[q] - base;
@@ -139,103 +161,84 @@ __device__ __forceinline__ int l2l_kc_begin(int rt, int R)
     return (2 * tri_count(jmin)) / 4;
 }
 
-// The block's columns (slot x component) and each slot's child per octant.
-struct ShiftTile {
-    int node[kShiftCols];                 // parent node of column c (-1 past the end)
-    int b[kShiftCols];                    // charge component of column c
-    int kid[kShiftCols][8];               // child node of column c's parent per octant (-1 absent)
-};
-
-// Columns [(blockIdx.x * per + h) * 32, + 32): part h of the block's per x 32 columns.
-__device__ void shift_tile(ShiftTile& t, const int32_t* __restrict__ list, int32_t slot0, int64_t ncols, int qd,
-                           const int32_t* __restrict__ child_beg, const int32_t* __restrict__ nchild,
-                           const uint64_t* __restrict__ key, int per = 1, int h = 0)
-{
-    const int64_t c0 = (int64_t(blockIdx.x) * per + h) * kShiftCols;
-    for (int c = threadIdx.x; c < kShiftCols; c += blockDim.x) {
-        const int64_t col = c0 + c;
-        for (int o = 0; o < 8; ++o) t.kid[c][o] = -1;
-        if (col < ncols) {
-            const int64_t s = col / qd;
-            const int g = list[slot0 + s];
-            t.node[c] = g;
-            t.b[c] = static_cast<int>(col - s * qd);
-            const int cb = child_beg[g], nc = nchild[g];
-            for (int k = cb; k < cb + nc; ++k) t.kid[c][key[k] & 7] = k;
-        } else {
-            t.node[c] = -1;
-            t.b[c] = 0;
-        }
-    }
-}
-
-// M2M into the parents of one level: columns [blockIdx.x * 32, + 32) of the
-// ncols = slots x qd columns; op = that level's OpM fragments.
+// M2M into the parents of one level: columns [blockIdx.x * 16, + 16) of the
+// ncols = slots x qd columns, row tiles [blockIdx.y * 4, + 4); op = that
+// level's OpM fragments.
 __global__ void __launch_bounds__(32 * kShiftWarps) k_m2m_mma(const double* __restrict__ op, int R,
-                                                              const int32_t* __restrict__ list, int32_t slot0,
-                                                              int64_t ncols, int qd, const int32_t* __restrict__ child_beg,
-                                                              const int32_t* __restrict__ nchild,
-                                                              const uint64_t* __restrict__ key, double* __restrict__ M)
+                                                              const int32_t* __restrict__ list, const int32_t* __restrict__ kid,
+                                                              int32_t slot0, int64_t ncols, int qd, double* __restrict__ M)
 {
-    constexpr int kMaxRowTiles = 5;       // R / 8 / warps: R <= 306 (p <= 16)
-    __shared__ ShiftTile tile;
-    extern __shared__ double Bs[];        // [32 cols][LD]
-    const int RT = cdiv(R, 8), KC = cdiv(R, 4), LD = shift_ld(4 * KC);
-    // this block's share of the R output rows: row tiles [rt0, rt1)
-    const int per = cdiv(RT, gridDim.y), rt0 = blockIdx.y * per, rt1 = min(RT, rt0 + per);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lr = lane >> 2, lc = lane & 3;
-    shift_tile(tile, list, slot0, ncols, qd, child_beg, nchild, key);
-    double acc[kMaxRowTiles][4][2];
+    __shared__ double part[kShiftWarps][kM2MRows][kM2MTiles][2][32];
+    const int RT = cdiv(R, 8), KC = cdiv(R, 4), rt0 = blockIdx.y * kM2MRows;
+    const int lane = threadIdx.x & 31, oct = threadIdx.x >> 5, lr = lane >> 2, lc = lane & 3;
+    const int64_t c0 = int64_t(blockIdx.x) * (8 * kM2MTiles);
+    // the children of the warp's octant: column 8 q + lr
+    const double* src[kM2MTiles];
+    bool any = false;
 #pragma unroll
-    for (int j = 0; j < kMaxRowTiles; ++j)
+    for (int q = 0; q < kM2MTiles; ++q) {
+        const int64_t col = c0 + 8 * q + lr, s = col / qd;
+        const int k = col < ncols ? kid[8 * (slot0 + s) + oct] : -1;
+        src[q] = k >= 0 ? M + (int64_t(k) * qd + (col - s * qd)) * R : nullptr;
+        any |= k >= 0;
+    }
+    int kce[kM2MRows], kmax = 0;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) acc[j][q][0] = acc[j][q][1] = 0.0;
-    for (int oct = 0; oct < 8; ++oct) {
-        __syncthreads();                  // the tile is set / the previous octant's operands are consumed
-        for (int e = threadIdx.x; e < kShiftCols * LD; e += blockDim.x) {
-            const int c = e / LD, k = e - c * LD;
-            const int kid = tile.kid[c][oct];
-            Bs[e] = (k < R && kid >= 0) ? M[(int64_t(kid) * qd + tile.b[c]) * R + k] : 0.0;
-        }
-        __syncthreads();
-        const double* fo = op + int64_t(oct) * RT * KC * 32 + lane;
+    for (int j = 0; j < kM2MRows; ++j) {
+        kce[j] = rt0 + j < RT ? m2m_kc_end(rt0 + j, R) : 0;
+        kmax = max(kmax, kce[j]);
+    }
+    if (!__any_sync(0xffffffffu, any)) kmax = 0;
+    double acc[kM2MRows][kM2MTiles][2] = {};
+    const double* fr = op + (int64_t(oct) * RT + rt0) * KC * 32 + lane;
+    // operands kAhead K chunks ahead of their products
+    constexpr int kAhead = 4;
+    double a[kAhead][kM2MRows], b[kAhead][kM2MTiles];
+    auto fetch = [&](int kc, double (&fa)[kM2MRows], double (&fb)[kM2MTiles]) {
 #pragma unroll
-        for (int j = 0; j < kMaxRowTiles; ++j) {
-            const int rt = rt0 + warp + kShiftWarps * j;
-            if (rt >= rt1) break;
-            const double* fr = fo + int64_t(rt) * KC * 32;
-            const int kce = m2m_kc_end(rt, R);
-            // operator fragments four K chunks ahead of their products
-            double a4[4];
+        for (int j = 0; j < kM2MRows; ++j) fa[j] = kc < kce[j] ? __ldg(fr + (int64_t(j) * KC + kc) * 32) : 0.0;
+        const int r = 4 * kc + lc;
 #pragma unroll
-            for (int u = 0; u < 4; ++u) a4[u] = u < kce ? __ldg(fr + u * 32) : 0.0;
-            for (int kc = 0; kc < kce; kc += 4) {
+        for (int q = 0; q < kM2MTiles; ++q) fb[q] = kc < kmax && src[q] && r < R ? src[q][r] : 0.0;
+    };
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const double a = a4[u];
-                    a4[u] = kc + 4 + u < kce ? __ldg(fr + (kc + 4 + u) * 32) : 0.0;
-                    if (kc + u < kce) {
+    for (int u = 0; u < kAhead; ++u) fetch(u, a[u], b[u]);
+    for (int kc = 0; kc < kmax; kc += kAhead) {
 #pragma unroll
-                        for (int q = 0; q < 4; ++q)
-                            mma884(acc[j][q][0], acc[j][q][1], a, Bs[(q * 8 + lr) * LD + 4 * (kc + u) + lc]);
-                    }
+        for (int u = 0; u < kAhead; ++u) {
+            if (kc + u >= kmax) break;
+            double ca[kM2MRows], cb[kM2MTiles];
+#pragma unroll
+            for (int j = 0; j < kM2MRows; ++j) ca[j] = a[u][j];
+#pragma unroll
+            for (int q = 0; q < kM2MTiles; ++q) cb[q] = b[u][q];
+            fetch(kc + kAhead + u, a[u], b[u]);
+#pragma unroll
+            for (int j = 0; j < kM2MRows; ++j)
+                if (kc + u < kce[j]) {
+#pragma unroll
+                    for (int q = 0; q < kM2MTiles; ++q) mma884(acc[j][q][0], acc[j][q][1], ca[j], cb[q]);
                 }
-            }
         }
     }
 #pragma unroll
-    for (int j = 0; j < kMaxRowTiles; ++j) {
-        const int rt = rt0 + warp + kShiftWarps * j;
-        if (rt >= rt1) break;
-        const int r = 8 * rt + lr;
-        if (r >= R) continue;
+    for (int j = 0; j < kM2MRows; ++j)
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
+        for (int q = 0; q < kM2MTiles; ++q)
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int c = q * 8 + 2 * lc + h;
-                if (tile.node[c] >= 0) M[(int64_t(tile.node[c]) * qd + tile.b[c]) * R + r] = acc[j][q][h];
-            }
+            for (int h = 0; h < 2; ++h) part[oct][j][q][h][lane] = acc[j][q][h];
+    __syncthreads();
+    // octant sums in octant order; element (row 8 j + lr, column 8 q + 2 lc + h)
+    for (int e = threadIdx.x; e < kM2MRows * kM2MTiles * 64; e += 32 * kShiftWarps) {
+        const int l = e & 31, h = (e >> 5) & 1, q = (e >> 6) % kM2MTiles, j = (e >> 6) / kM2MTiles;
+        const int r = 8 * (rt0 + j) + (l >> 2);
+        const int64_t col = c0 + 8 * q + 2 * (l & 3) + h;
+        if (r >= R || col >= ncols) continue;
+        double v = 0.0;
+#pragma unroll
+        for (int o = 0; o < 8; ++o) v += part[o][j][q][h][l];
+        const int64_t s = col / qd;
+        M[(int64_t(list[slot0 + s]) * qd + (col - s * qd)) * R + r] = v;
     }
 }
 
@@ -249,24 +252,20 @@ struct L2LSide {
 
 template<int NQ>                          // NQ 8-column MMA tiles: 8 NQ columns per block
 __global__ void __launch_bounds__(32 * kShiftWarps) k_l2l_mma(L2LSide sa, L2LSide sb, const int32_t* __restrict__ list,
-                                                              int32_t slot0, int64_t ncols, int qd,
-                                                              const int32_t* __restrict__ child_beg,
-                                                              const int32_t* __restrict__ nchild,
-                                                              const uint64_t* __restrict__ key)
+                                                              const int32_t* __restrict__ kid, int32_t slot0, int64_t ncols, int qd)
 {
-    constexpr int NC = 8 * NQ;
+    constexpr int NC = 8 * NQ, kAhead = NQ > 2 ? 4 : 8;
     const L2LSide sd = blockIdx.y ? sb : sa;
     if (!sd.L) return;
-    __shared__ ShiftTile tile[NQ / 4];
     extern __shared__ double Bs[];        // [NC cols][LD]
     const int R = sd.R, RT8 = R, KC = cdiv(R, 4), LD = shift_ld(4 * KC);   // 8R rows: R row tiles
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lr = lane >> 2, lc = lane & 3;
-    for (int h = 0; h < NQ / 4; ++h) shift_tile(tile[h], list, slot0, ncols, qd, child_beg, nchild, key, NQ / 4, h);
-    __syncthreads();
-    for (int e = threadIdx.x; e < NC * LD; e += blockDim.x) {
-        const int c = e / LD, k = e - c * LD;
-        const int g = tile[c / kShiftCols].node[c % kShiftCols];
-        Bs[e] = (k < R && g >= 0) ? sd.L[(int64_t(g) * qd + tile[c / kShiftCols].b[c % kShiftCols]) * R + k] : 0.0;
+    const int64_t c0 = int64_t(blockIdx.x) * NC;
+    // a warp per column: its parent's local, zero padding
+    for (int c = warp; c < NC; c += kShiftWarps) {
+        const int64_t col = c0 + c, s = col / qd;
+        const double* src = col < ncols ? sd.L + (int64_t(list[slot0 + s]) * qd + (col - s * qd)) * R : nullptr;
+        for (int k = lane; k < LD; k += 32) Bs[c * LD + k] = src && k < R ? src[k] : 0.0;
     }
     __syncthreads();
     // this block's share of the 8R output rows: row tiles [rt0, rt1)
@@ -275,15 +274,15 @@ __global__ void __launch_bounds__(32 * kShiftWarps) k_l2l_mma(L2LSide sa, L2LSid
         double acc[NQ][2] = {};
         const double* fr = sd.op + int64_t(rt) * KC * 32 + lane;
         const int kcb = l2l_kc_begin(rt, R);
-        // operator fragments four K chunks ahead of their products
-        double a4[4];
+        // operator fragments kAhead K chunks ahead of their products
+        double a4[kAhead];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) a4[u] = kcb + u < KC ? __ldg(fr + (kcb + u) * 32) : 0.0;
-        for (int kc = kcb; kc < KC; kc += 4) {
+        for (int u = 0; u < kAhead; ++u) a4[u] = kcb + u < KC ? __ldg(fr + (kcb + u) * 32) : 0.0;
+        for (int kc = kcb; kc < KC; kc += kAhead) {
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
+            for (int u = 0; u < kAhead; ++u) {
                 const double a = a4[u];
-                a4[u] = kc + 4 + u < KC ? __ldg(fr + (kc + 4 + u) * 32) : 0.0;
+                a4[u] = kc + kAhead + u < KC ? __ldg(fr + (kc + kAhead + u) * 32) : 0.0;
                 if (kc + u < KC) {
 #pragma unroll
                     for (int q = 0; q < NQ; ++q)
@@ -296,11 +295,9 @@ __global__ void __launch_bounds__(32 * kShiftWarps) k_l2l_mma(L2LSide sa, L2LSid
         for (int q = 0; q < NQ; ++q)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const int c = q * 8 + 2 * lc + h;
-                const ShiftTile& t = tile[c / kShiftCols];
-                const int cc = c % kShiftCols;
-                const int kid = t.node[cc] >= 0 ? t.kid[cc][oct] : -1;
-                if (kid >= 0) sd.L[(int64_t(kid) * qd + t.b[cc]) * R + i] += acc[q][h];
+                const int64_t col = c0 + q * 8 + 2 * lc + h, s = col / qd;
+                const int k = col < ncols ? kid[8 * (slot0 + s) + oct] : -1;
+                if (k >= 0) sd.L[(int64_t(k) * qd + (col - s * qd)) * R + i] += acc[q][h];
             }
     }
 }
@@ -393,6 +390,7 @@ void shift_setup(Plan& pl)
     flag.alloc(n, st);
     pl.sh_slot.alloc(n + 1, st);                        // exclusive scans write n + 1 entries
     pl.sh_list.alloc(std::max<int64_t>(n, 1), st);
+    pl.sh_kid.alloc(std::max<int64_t>(8 * n, 1), st);
     k_has_children<<<grid_for(n, c.sm_count), 256, 0, st>>>(t.nchild.ptr, base, n, flag.ptr);
     SFMM_CHECK_LAUNCH();
     exclusive_scan_i32(flag.ptr, pl.sh_slot.ptr, n, st);
@@ -401,7 +399,8 @@ void shift_setup(Plan& pl)
     SFMM_CUDA(cudaMemcpyAsync(lvl.ptr, t.lvl_off.data(), t.lvl_off.size() * sizeof(int64_t), cudaMemcpyHostToDevice, st));
     DevBuf<int32_t> S;
     S.alloc(t.depth + 1, st);
-    k_slots<<<grid_for(n, c.sm_count), 256, 0, st>>>(flag.ptr, pl.sh_slot.ptr, base, n, pl.sh_list.ptr, lvl.ptr, t.depth, S.ptr);
+    k_slots<<<grid_for(n, c.sm_count), 256, 0, st>>>(flag.ptr, pl.sh_slot.ptr, base, n, t.child_beg.ptr, t.nchild.ptr,
+                                                       t.key.ptr, pl.sh_list.ptr, pl.sh_kid.ptr, lvl.ptr, t.depth, S.ptr);
     SFMM_CHECK_LAUNCH();
     pl.sh_S.assign(t.depth + 1, 0);
     SFMM_CUDA(cudaMemcpyAsync(pl.sh_S.data(), S.ptr, (t.depth + 1) * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
@@ -419,9 +418,9 @@ void shift_setup(Plan& pl)
                                                                           RB, pl.sh_ops.ptr);
     SFMM_CHECK_LAUNCH();
     const size_t smem = size_t(8 * kL2LTiles) * shift_ld(4 * cdiv(RB, 4)) * sizeof(double);
-    SFMM_REQUIRE(smem + 2 * sizeof(ShiftTile) <= 227 * 1024, FMM_ERR_UNSUPPORTED, "shift operands exceed shared memory");
-    allow_max_smem(k_m2m_mma);
+    SFMM_REQUIRE(smem <= 227 * 1024, FMM_ERR_UNSUPPORTED, "shift operands exceed shared memory");
     allow_max_smem(k_l2l_mma<kL2LTiles>);
+    allow_max_smem(k_l2l_mma<kL2LSmallTiles>);
     pl.shift_on = true;
 }
 
@@ -436,10 +435,9 @@ void shift_m2m(Plan& pl, const EvalArgs& a, int lp, cudaStream_t st)
     const int64_t per_level = (m2m_frags(R) + l2l_frags(R) + l2l_frags(2 * pl.T1)) * 32;
     const double* op = pl.sh_ops.ptr + per_level * (lc - 3);
     const int64_t ncols = n * qd;
-    const size_t smem = size_t(kShiftCols) * shift_ld(4 * cdiv(R, 4)) * sizeof(double);
-    k_m2m_mma<<<dim3(static_cast<unsigned>((ncols + kShiftCols - 1) / kShiftCols), kM2MRowGroups), 32 * kShiftWarps, smem,
-                st>>>(
-        op, R, pl.sh_list.ptr, slot0, ncols, qd, t.child_beg.ptr, t.nchild.ptr, t.key.ptr, reinterpret_cast<double*>(a.M));
+    constexpr int NC = 8 * kM2MTiles;
+    k_m2m_mma<<<dim3(static_cast<unsigned>((ncols + NC - 1) / NC), cdiv(cdiv(R, 8), kM2MRows)), 32 * kShiftWarps, 0, st>>>(
+        op, R, pl.sh_list.ptr, pl.sh_kid.ptr, slot0, ncols, qd, reinterpret_cast<double*>(a.M));
     SFMM_CHECK_LAUNCH();
 }
 
@@ -455,15 +453,18 @@ void shift_l2l(Plan& pl, const EvalArgs& a, int lc, cudaStream_t st)
     const L2LSide sa{op + m2m_frags(RA) * 32, RA, a.want_pot ? reinterpret_cast<double*>(a.LA) : nullptr};
     const L2LSide sb{op + (m2m_frags(RA) + l2l_frags(RA)) * 32, RB, a.want_field ? reinterpret_cast<double*>(a.LB) : nullptr};
     const int64_t ncols = n * qd;
-    constexpr int NC = 8 * kL2LTiles;
-    const size_t smem = size_t(NC) * shift_ld(4 * cdiv(RB, 4)) * sizeof(double);
-    // small levels (few column tiles) split their rows over more blocks so
-    // the level still spreads over the SMs (each block keeps >= 8 row tiles)
-    const int64_t ctiles = (ncols + NC - 1) / NC;
-    const int rg = static_cast<int>(std::min<int64_t>(std::max<int64_t>(kL2LRowGroups, int64_t(t.ctx->sm_count) / ctiles),
-                                                      std::max(1, RA / kShiftWarps)));
-    k_l2l_mma<kL2LTiles><<<dim3(static_cast<unsigned>(ctiles), 2, static_cast<unsigned>(rg)), 32 * kShiftWarps, smem, st>>>(
-        sa, sb, pl.sh_list.ptr, slot0, ncols, qd, t.child_beg.ptr, t.nchild.ptr, t.key.ptr);
+    // small levels (too few column tiles for the SMs even with their rows split)
+    // take narrow tiles and a row tile per warp
+    const int64_t ctiles = (ncols + 8 * kL2LTiles - 1) / (8 * kL2LTiles);
+    auto launch = [&](auto tiles, int64_t rg) {
+        constexpr int NQ = decltype(tiles)::value, NC = 8 * NQ;
+        const size_t smem = size_t(NC) * shift_ld(4 * cdiv(RB, 4)) * sizeof(double);
+        k_l2l_mma<NQ><<<dim3(static_cast<unsigned>((ncols + NC - 1) / NC), 2, static_cast<unsigned>(rg)), 32 * kShiftWarps, smem, st>>>(
+            sa, sb, pl.sh_list.ptr, pl.sh_kid.ptr, slot0, ncols, qd);
+    };
+    const int64_t sms = t.ctx->sm_count;
+    if (ctiles * 2 * kL2LRowGroups < 2 * sms) launch(std::integral_constant<int, kL2LSmallTiles>{}, cdiv(RB, kShiftWarps));
+    else launch(std::integral_constant<int, kL2LTiles>{}, std::min<int64_t>(std::max<int64_t>(kL2LRowGroups, sms / ctiles), std::max(1, RA / kShiftWarps)));
     SFMM_CHECK_LAUNCH();
 }
 
