@@ -585,41 +585,57 @@ __global__ void k_nlist(int level, LevelTabs L, const uint64_t* __restrict__ key
 // The refinement above, the colleague lists and the leaf numbering in ONE
 // cooperative launch (every block resident at once), the steps separated by
 // grid barriers instead of kernel boundaries and host reads of counts.  Per
-// level (S splitting nodes in `sp`, T tiles of at most kWTile points):
-//   A  colleagues of the level's nodes; tile counts of the splitting nodes,
-//      one partial sum per block over its contiguous range of nodes
-//   B  tile offsets (each block adds up the partials before its range); T
-//   C  digit histogram of every tile (a warp per tile, tiles in contiguous
-//      ranges per block), the block's per-digit totals, and per-node digit
-//      counts by integer atomics (exact whatever the order)
+// level (S splitting nodes in `sp`, T tiles of at most a.tile points):
+//   C  colleagues of the level's nodes (a warp per parent); digit histogram of
+//      every tile (a warp per tile, tiles in contiguous ranges per block), the
+//      block's per-digit totals, and per-node digit counts by integer atomics
+//      (exact whatever the order)
 //   D  per-digit exclusive prefixes over the tiles (the [digit][tile] scan of
-//      the level path, row by row); child counts per node, block totals
-//   E  child numbering, the children's node fields, and the stable scatter:
-//      a warp takes a tile's points in index order, 32 at a time, and places
-//      each after the earlier points of its digit (match + 8 ballots)
-// and after the last level the leaf numbering (two steps).  The partition,
-// node numbering and lists are the level path's, bit for bit.
+//      the level path, row by row); child, splitting-child and next-level tile
+//      counts per node, block totals
+//   E  child numbering, the children's node fields, the next level's tile
+//      offsets, and the stable scatter: a warp takes a tile's points in index
+//      order, 32 at a time, and places each after the earlier points of its
+//      digit (4 ballots give every digit's lane mask)
+// and after the last level the leaf numbering (two steps).  A level whose
+// splitting nodes are one tile each (all but the upper ones) has every count
+// of D in the warp that took the histogram, so D and its barrier are left out.
+// The partition, node numbering and lists are the level path's, bit for bit.
 //
-// A level that needs more node slots than allocated ends the launch at its
-// start with kRefGrow; the host grows the node arrays and launches again from
-// that level.  Each barrier wait is bounded (%globaltimer, about two seconds,
-// and an iteration cap); a wait that runs out sets an abort flag that every
-// other waiting block sees, and the launch ends with kRefTimeout.
+// Small trees are bound by the chain of barriers and dependent loads, not by
+// bandwidth: the step count and each step's latency are what this layout cuts.
+// Measured against five barriers a level, 1024-point tiles, a warp per node for
+// the colleagues and a barrier of three round trips: 2k points 204 -> 71 us,
+// 100k 225 -> 79, 400k (two clusters) 460 -> 174, 1M 650 -> 279; at 16M, where
+// the passes over keys and indices count, 1972 -> 1219.
+//
+// A level that needs more node slots than allocated ends the launch before its
+// children are numbered with kRefGrow; the host grows the node arrays and
+// launches again, and the launch resumes at step E of that level.  Each
+// barrier wait is bounded (%globaltimer, about two seconds, and an iteration
+// cap); a wait that runs out sets an abort flag that every other waiting block
+// sees, and the launch ends with kRefTimeout.
 constexpr int kRefThreads = 256;
 constexpr int kRefWarps = kRefThreads / 32;
-constexpr int kWTile = 1024;                  // points per tile (one warp)
-constexpr int kParts = 12;                    // partial sums per block
+// Points per tile (one warp): a tile is a serial chain, so its length is
+// latency.  1024 points from 4 Mi points on, where the 4,736 warps of a full
+// grid (148 SMs x 4 blocks) about fill with such tiles and fewer tiles mean
+// shorter prefix scans and fewer atomics; below, 256.
+constexpr int kTileSmall = 256, kTileLarge = 1024;
+constexpr int64_t kTileLargeFrom = 4 << 20;
+constexpr int kParts = 16;                    // partial sums per block
+constexpr int kPartDigit = 1, kPartCount = 9, kPartLeaf = 12;
 constexpr unsigned long long kBarrierNs = 2000000000ull;
 
 enum { kRefDone = 0, kRefGrow = 1, kRefTimeout = 2, kRefOverflow = 3 };
 
 struct RefineState {
     unsigned bar_count;
-    unsigned bar_gen;
     int abort;
     int status;
+    int resume;                      // start at step E (after kRefGrow)
     int level;                       // level whose splitting nodes come next
-    int S;                           // their number
+    int S, T;                        // their number, their tiles
     int cur;                         // which sp / point buffers hold them
     int need;                        // children of that level (kRefGrow)
     int gate;                        // set by nothing: the wait of the stall test
@@ -631,12 +647,14 @@ struct RefineState {
 struct RefineArgs {
     uint64_t* key;
     int32_t *pbeg, *pend, *parent, *child_beg, *nchild, *col, *leaf_id, *leaf_node;
+    int32_t* cmask;                  // octants present, 0 for a leaf
     long long cap;
     uint64_t* pkey[2];
     int32_t* pord[2];
     int32_t* final_ord;
-    int32_t* sp[2];
-    int32_t *tile_off, *hist, *pre, *ncnt, *offs, *nch, *nsp, *part;
+    int32_t *sp[2], *tile_off[2], *ncnt[2];
+    int32_t *hist, *pre, *offs, *nst, *ntl, *part;
+    int tile;
     int smax, tmax;
     int max_level, ppn;
     int stall;                       // test switch: block 0 waits on `gate` (never set)
@@ -657,44 +675,37 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p)
     return v;
 }
 
-__device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v)
-{
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-// Grid barrier (sense by generation).  Returns false when this block must
-// leave: its wait ran out or another block's did.
-__device__ bool grid_barrier(RefineState* st)
+// Grid barrier number `phase` of this launch: the arrivals are counted up and
+// never reset, so the last arrival itself is what the others wait for.  Returns
+// false when this block must leave: its wait ran out or another block's did
+// (that block never arrives again, so every later wait ends here too).
+__device__ bool grid_barrier(RefineState* st, unsigned& phase)
 {
     __shared__ int s_ok;
+    ++phase;
     __syncthreads();
     if (threadIdx.x == 0) {
         int ok = 1;
-        volatile int* abort = &st->abort;
-        if (*abort) {
-            ok = 0;
-        } else {
-            const unsigned gen = ld_acquire_u32(&st->bar_gen);
-            __threadfence();
-            if (atomicAdd(&st->bar_count, 1u) == gridDim.x - 1) {
-                atomicExch(&st->bar_count, 0u);
-                __threadfence();
-                st_release_u32(&st->bar_gen, gen + 1);
-            } else {
-                const unsigned long long t0 = global_ns();
-                unsigned spins = 0, nap = 32;
-                while (ld_acquire_u32(&st->bar_gen) == gen) {
-                    if (*abort || ++spins > (1u << 25) || global_ns() - t0 > kBarrierNs) {
+        const unsigned target = phase * gridDim.x;
+        __threadfence();
+        if (atomicAdd(&st->bar_count, 1u) + 1 != target) {
+            volatile int* abort = &st->abort;
+            unsigned long long t0 = 0;
+            unsigned spins = 0;
+            while (static_cast<int>(ld_acquire_u32(&st->bar_count) - target) < 0) {
+                if ((++spins & 15u) == 0) {
+                    const unsigned long long now = global_ns();
+                    if (!t0) t0 = now;
+                    if (*abort || spins > (1u << 25) || now - t0 > kBarrierNs) {
                         atomicExch(&st->abort, 1);
                         ok = 0;
                         break;
                     }
-                    __nanosleep(nap);
-                    if (nap < 256) nap *= 2;
+                    if (spins >= 64) __nanosleep(64);
                 }
             }
-            __threadfence();
         }
+        __threadfence();
         s_ok = ok;
     }
     __syncthreads();
@@ -713,20 +724,15 @@ __device__ int block_excl(int v, int* tot, int* sh)
     }
     if (lane == 31) sh[w] = x;
     __syncthreads();
-    if (w == 0) {
-        int y = lane < kRefWarps ? sh[lane] : 0;
+    int before = 0, all = 0;
 #pragma unroll
-        for (int o = 1; o < kRefWarps; o <<= 1) {
-            const int z = __shfl_up_sync(0xffffffffu, y, o);
-            if (lane >= o) y += z;
-        }
-        if (lane < kRefWarps) sh[lane] = y;
+    for (int k = 0; k < kRefWarps; ++k) {
+        if (k < w) before += sh[k];
+        all += sh[k];
     }
+    *tot = all;
     __syncthreads();
-    const int before = (w ? sh[w - 1] : 0) + x - v;
-    *tot = sh[kRefWarps - 1];
-    __syncthreads();
-    return before;
+    return before + x - v;
 }
 
 __device__ int block_sum(int v, int* sh)
@@ -736,24 +742,37 @@ __device__ int block_sum(int v, int* sh)
     return tot;
 }
 
-// Field f of the per-block partials: the sum over blocks before this one and
-// over all blocks.
-__device__ void parts_sums(const int32_t* part, int f, int* before, int* all, int* sh)
+// Fields f .. f + N - 1 of the per-block partials: the sums over the blocks
+// before this one and over all blocks.
+template<int N>
+__device__ void parts_sums(const int32_t* part, int f, int* before, int* all, int (*sh)[kRefWarps])
 {
-    int x = 0, y = 0;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int v[2 * N] = {};
     for (int k = threadIdx.x; k < static_cast<int>(gridDim.x); k += blockDim.x) {
-        const int v = part[k * kParts + f];
-        y += v;
-        if (k < static_cast<int>(blockIdx.x)) x += v;
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const int x = part[k * kParts + f + i];
+            v[N + i] += x;
+            if (k < static_cast<int>(blockIdx.x)) v[i] += x;
+        }
     }
-    *before = block_sum(x, sh);
-    *all = block_sum(y, sh);
-}
-
-__device__ __forceinline__ int tile_count(const RefineArgs& a, const int32_t* sp, int s)
-{
-    const int g = sp[s];
-    return (a.pend[g] - a.pbeg[g] + kWTile - 1) / kWTile;
+#pragma unroll
+    for (int i = 0; i < 2 * N; ++i) {
+        v[i] = __reduce_add_sync(0xffffffffu, v[i]);
+        if (lane == 0) sh[i][w] = v[i];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        before[i] = all[i] = 0;
+#pragma unroll
+        for (int k = 0; k < kRefWarps; ++k) {
+            before[i] += sh[i][k];
+            all[i] += sh[N + i][k];
+        }
+    }
+    __syncthreads();
 }
 
 // first tile of the warp: binary search; later (larger) tiles: walk on
@@ -764,16 +783,25 @@ __device__ __forceinline__ int seg_of(const int32_t* tile_off, int S, int t, int
     return s;
 }
 
-__global__ void __launch_bounds__(kRefThreads) k_refine(RefineArgs a)
+// lanes of the warp whose point has octant d, from the ballots of the three
+// bits and of the lanes that hold a point
+__device__ __forceinline__ unsigned octant_lanes(int d, unsigned b0, unsigned b1, unsigned b2, unsigned valid)
 {
-    __shared__ int sh[kRefWarps];
-    __shared__ int s_dig[8];
+    return valid & (d & 1 ? b0 : ~b0) & (d & 2 ? b1 : ~b1) & (d & 4 ? b2 : ~b2);
+}
+
+__global__ void __launch_bounds__(kRefThreads, 4) k_refine(RefineArgs a)
+{
+    __shared__ int sh[kRefWarps], sh6[6][kRefWarps];
+    __shared__ int s_dig[8], s_cnt[3];
     __shared__ long long s_lvl[kKeyLevel + 3];
     RefineState* st = a.st;
     const int G = gridDim.x, b = blockIdx.x, tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
     const unsigned lt = (1u << lane) - 1u;
-    const int64_t gthreads = int64_t(G) * kRefThreads, gtid = int64_t(b) * kRefThreads + tid;
+    const int gwarp = b * kRefWarps + warp, gwarps = G * kRefWarps;
+    const int tile = a.tile;
+    unsigned phase = 0;
     if (a.stall && b == 0) {
         // test of the bounded waits: block 0 never reaches the first barrier;
         // its thread 0 waits on a flag nothing sets, then raises the abort
@@ -789,240 +817,267 @@ __global__ void __launch_bounds__(kRefThreads) k_refine(RefineArgs a)
         }
         return;
     }
-    int level = st->level, S = st->S, cur = st->cur;
-    int64_t lo = st->lvl_off[level], total = st->total;
+    int level = st->level, S = st->S, T = st->T, cur = st->cur, Sprev = 0;
+    bool resume = st->resume != 0;
+    int64_t total = st->total;
     int status = kRefDone, need = 0;
 
     for (;;) {
-        const int32_t* sp = cur ? a.sp[1] : a.sp[0];
-        int32_t* spn = cur ? a.sp[0] : a.sp[1];
-        const uint64_t* kin = cur ? a.pkey[1] : a.pkey[0];
-        uint64_t* kout = cur ? a.pkey[0] : a.pkey[1];
-        const int32_t* oin = cur ? a.pord[1] : a.pord[0];
-        int32_t* oout = cur ? a.pord[0] : a.pord[1];
+        const int32_t* sp = a.sp[cur];
+        int32_t* spn = a.sp[cur ^ 1];                     // before E: the splitting nodes of the level above
+        const int32_t* tile_off = a.tile_off[cur];
+        int32_t* tile_next = a.tile_off[cur ^ 1];
+        int32_t* ncnt = a.ncnt[cur];
+        int32_t* ncnt_next = a.ncnt[cur ^ 1];
+        const uint64_t* kin = a.pkey[cur];
+        uint64_t* kout = a.pkey[cur ^ 1];
+        const int32_t* oin = a.pord[cur];
+        int32_t* oout = a.pord[cur ^ 1];
         const int child_may_split = (level + 1) < a.max_level;
-
-        // ---- A: colleagues of this level (a warp per node, a lane per
-        //      neighbour of the parent); tile counts
-        for (int64_t g = lo + (gtid >> 5); g < total; g += gthreads >> 5) {
-            int32_t* my = a.col + 27 * g;
-            if (lane < 27) my[lane] = (level == 0 && lane == 13) ? static_cast<int32_t>(g) : -1;
-            if (level == 0) continue;
-            __syncwarp();
-            const I3 me = key_ijk(a.key[g]);
-            const int P = lane < 27 ? a.col[27 * int64_t(a.parent[g]) + lane] : -1;
-            if (P >= 0) {
-                const int cb = a.child_beg[P], nc = a.nchild[P];
-                uint64_t kc[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) kc[j] = j < nc ? a.key[cb + j] : 0;
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    if (j >= nc) break;
-                    const I3 o = key_ijk(kc[j]);
-                    const int dx = o.x - me.x, dy = o.y - me.y, dz = o.z - me.z;
-                    if (abs(dx) <= 1 && abs(dy) <= 1 && abs(dz) <= 1) my[slot_of(dx, dy, dz)] = cb + j;
-                }
-            }
-            __syncwarp();
-        }
-        if (S == 0) break;
-        const int cs = (S + G - 1) / G, s0 = min(S, b * cs), s1 = min(S, s0 + cs);
-        {
-            int mine = 0;
-            for (int s = s0 + tid; s < s1; s += kRefThreads) {
-                mine += tile_count(a, sp, s);
-#pragma unroll
-                for (int d = 0; d < 8; ++d) a.ncnt[8 * s + d] = 0;
-            }
-            const int tot = block_sum(mine, sh);
-            if (tid == 0) a.part[b * kParts] = tot;
-        }
-        if (!grid_barrier(st)) return;
-
-        // ---- B: tile offsets
-        int T;
-        {
-            int before;
-            parts_sums(a.part, 0, &before, &T, sh);
-            if (T > a.tmax) {
-                status = kRefOverflow;
-                break;
-            }
-            int carry = before;
-            for (int base = s0; base < s1; base += kRefThreads) {
-                const int s = base + tid;
-                const int v = s < s1 ? tile_count(a, sp, s) : 0;
-                int tot;
-                const int ex = block_excl(v, &tot, sh);
-                if (s < s1) a.tile_off[s] = carry + ex;
-                carry += tot;
-            }
-        }
-        if (!grid_barrier(st)) return;
-
-        // ---- C: digit histograms
         const int shift = 3 * (kKeyLevel - 1 - level);
+        const bool flat = T == S;                         // one tile per splitting node
         const int ct = (T + G - 1) / G, t0 = min(T, b * ct), t1 = min(T, t0 + ct);
-        if (tid < 8) s_dig[tid] = 0;
-        __syncthreads();
-        {
-            int s = -1;
-            for (int t = t0 + warp; t < t1; t += kRefWarps) {
-                s = seg_of(a.tile_off, S, t, s);
-                const int g = sp[s];
-                const int pb = a.pbeg[g] + (t - a.tile_off[s]) * kWTile;
-                const int pe = min(a.pend[g], pb + kWTile);
-                int c = 0;                                   // lane d < 8: points of digit d
-                for (int i0 = pb; i0 < pe; i0 += 128) {
-                    int dg[4];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const int i = i0 + 32 * u + lane;
-                        dg[u] = i < pe ? static_cast<int>((kin[i] >> shift) & 7) : 8;
-                    }
-#pragma unroll
-                    for (int u = 0; u < 4; ++u)
-#pragma unroll
-                        for (int d = 0; d < 8; ++d) {
-                            const unsigned m = __ballot_sync(0xffffffffu, dg[u] == d);
-                            if (lane == d) c += __popc(m);
-                        }
-                }
-                if (lane < 8) {
-                    a.hist[int64_t(lane) * T + t] = c;
-                    if (c) {
-                        atomicAdd(&a.ncnt[8 * s + lane], c);
-                        atomicAdd(&s_dig[lane], c);
-                    }
-                }
-            }
-        }
-        __syncthreads();
-        if (tid < 8) a.part[b * kParts + 1 + tid] = s_dig[tid];
-        if (!grid_barrier(st)) return;
+        const int cs = (S + G - 1) / G, s0 = min(S, b * cs), s1 = min(S, s0 + cs);
 
-        // ---- D: per-digit tile prefixes (warp d); node statistics
-        {
-            const int d = warp;                               // 8 warps, one per digit
-            int base = 0;
-            for (int k = lane; k < b; k += 32) base += a.part[k * kParts + 1 + d];
+        if (!resume) {
+            // ---- C: digit histograms
+            if (tid < 8) s_dig[tid] = 0;
+            if (tid < 3) s_cnt[tid] = 0;
+            __syncthreads();
+            {
+                int s = -1;
+                for (int t = t0 + warp; t < t1; t += kRefWarps) {
+                    s = flat ? t : seg_of(tile_off, S, t, s);
+                    const int g = sp[s];
+                    const int pb = a.pbeg[g] + (flat ? 0 : (t - tile_off[s]) * tile);
+                    const int pe = min(a.pend[g], pb + tile);
+                    int c = 0;                            // lane d < 8: points of digit d
+                    for (int i0 = pb; i0 < pe; i0 += 256) {
+                        int dg[8];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) base += __shfl_xor_sync(0xffffffffu, base, o);
-            for (int t = t0; t < t1; t += 32) {
-                const int tt = t + lane;
-                const int v = tt < t1 ? a.hist[int64_t(d) * T + tt] : 0;
-                int x = v;
+                        for (int u = 0; u < 8; ++u) {
+                            const int i = i0 + 32 * u + lane;
+                            dg[u] = i < pe ? static_cast<int>((kin[i] >> shift) & 7) : 8;
+                        }
 #pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int y = __shfl_up_sync(0xffffffffu, x, o);
-                    if (lane >= o) x += y;
+                        for (int u = 0; u < 8; ++u) {
+                            const unsigned b0 = __ballot_sync(0xffffffffu, dg[u] & 1);
+                            const unsigned b1 = __ballot_sync(0xffffffffu, dg[u] & 2);
+                            const unsigned b2 = __ballot_sync(0xffffffffu, dg[u] & 4);
+                            const unsigned v = __ballot_sync(0xffffffffu, dg[u] < 8);
+                            if (lane < 8) c += __popc(octant_lanes(lane, b0, b1, b2, v));
+                        }
+                    }
+                    if (flat) {
+                        // the whole node: its counts and the children's tiles
+                        int x = c;
+#pragma unroll
+                        for (int o = 1; o < 8; o <<= 1) {
+                            const int y = __shfl_up_sync(0xffffffffu, x, o);
+                            if (lane >= o) x += y;
+                        }
+                        const bool sp_d = c > a.ppn && child_may_split;
+                        const int nc = __popc(__ballot_sync(0xffffffffu, c > 0));
+                        const int ns = __popc(__ballot_sync(0xffffffffu, sp_d));
+                        const int nt = __reduce_add_sync(0xffffffffu, sp_d ? (c + tile - 1) / tile : 0);
+                        if (lane < 8) {
+                            ncnt[8 * s + lane] = c;
+                            a.offs[8 * s + lane] = x - c;
+                        }
+                        if (lane == 0) {
+                            a.nst[s] = nc | ns << 16;
+                            a.ntl[s] = nt;
+                            atomicAdd(&s_cnt[0], nc);
+                            atomicAdd(&s_cnt[1], ns);
+                            atomicAdd(&s_cnt[2], nt);
+                        }
+                    } else if (lane < 8) {
+                        a.hist[int64_t(lane) * T + t] = c;
+                        if (c) {
+                            atomicAdd(&ncnt[8 * s + lane], c);
+                            atomicAdd(&s_dig[lane], c);
+                        }
+                    }
                 }
-                if (tt < t1) a.pre[int64_t(d) * T + tt] = base + x - v;
-                base += __shfl_sync(0xffffffffu, x, 31);
+            }
+
+            // colleagues of this level: a warp per parent, lane k < 27 holding
+            // the parent's neighbour k (its first child and octants); the
+            // entry of child octant o at offset d is octant (o + d) & 1 of
+            // the neighbour floor((o + d) / 2), per axis
+            if (level == 0 && gwarp == 0 && lane < 27) a.col[lane] = lane == 13 ? 0 : -1;
+            const int ox = lane % 3 - 1, oy = lane / 3 % 3 - 1, oz = lane / 9 - 1;
+            for (int s = gwarps - 1 - gwarp; s < Sprev; s += gwarps) {
+                const int g = spn[s];
+                const int P = lane < 27 ? a.col[27 * int64_t(g) + lane] : -1;
+                const int cb = P >= 0 ? a.child_beg[P] : -1;
+                const int mask = P >= 0 ? a.cmask[P] : 0;
+                const int mine = __shfl_sync(0xffffffffu, mask, 13);
+                int h = __shfl_sync(0xffffffffu, cb, 13);
+                for (int o = 0; o < 8; ++o) {
+                    if (!((mine >> o) & 1)) continue;
+                    const int x = (o & 1) + ox, y = ((o >> 1) & 1) + oy, z = (o >> 2) + oz;
+                    const int from = slot_of(x >> 1, y >> 1, z >> 1);
+                    const int oct = (x & 1) | (y & 1) << 1 | (z & 1) << 2;
+                    const int m = __shfl_sync(0xffffffffu, mask, from & 31);
+                    const int f = __shfl_sync(0xffffffffu, cb, from & 31);
+                    if (lane < 27)
+                        a.col[27 * int64_t(h) + lane] = (m >> oct) & 1 ? f + __popc(m & ((1 << oct) - 1)) : -1;
+                    ++h;
+                }
+            }
+            if (S == 0) break;
+            __syncthreads();
+            if (flat) {
+                if (tid < 3) a.part[b * kParts + kPartCount + tid] = s_cnt[tid];
+            } else if (tid < 8) {
+                a.part[b * kParts + kPartDigit + tid] = s_dig[tid];
+            }
+            if (!grid_barrier(st, phase)) return;
+
+            // ---- D: per-digit tile prefixes (warp d); node statistics
+            if (!flat) {
+                {
+                    const int d = warp;                   // 8 warps, one per digit
+                    int base = 0;
+                    for (int k = lane; k < b; k += 32) base += a.part[k * kParts + kPartDigit + d];
+                    base = __reduce_add_sync(0xffffffffu, base);
+                    for (int t = t0; t < t1; t += 32) {
+                        const int tt = t + lane;
+                        const int v = tt < t1 ? a.hist[int64_t(d) * T + tt] : 0;
+                        int x = v;
+#pragma unroll
+                        for (int o = 1; o < 32; o <<= 1) {
+                            const int y = __shfl_up_sync(0xffffffffu, x, o);
+                            if (lane >= o) x += y;
+                        }
+                        if (tt < t1) a.pre[int64_t(d) * T + tt] = base + x - v;
+                        base += __shfl_sync(0xffffffffu, x, 31);
+                    }
+                }
+                int m[3] = {0, 0, 0};
+                for (int s = s0 + tid; s < s1; s += kRefThreads) {
+                    int off = 0, nc = 0, ns = 0, nt = 0;
+#pragma unroll
+                    for (int d = 0; d < 8; ++d) {
+                        const int c = ncnt[8 * s + d];
+                        a.offs[8 * s + d] = off;
+                        off += c;
+                        nc += c > 0;
+                        if (c > a.ppn && child_may_split) {
+                            ++ns;
+                            nt += (c + tile - 1) / tile;
+                        }
+                    }
+                    a.nst[s] = nc | ns << 16;
+                    a.ntl[s] = nt;
+                    m[0] += nc;
+                    m[1] += ns;
+                    m[2] += nt;
+                }
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    const int v = __reduce_add_sync(0xffffffffu, m[i]);
+                    if (lane == 0 && v) atomicAdd(&s_cnt[i], v);
+                }
+                __syncthreads();
+                if (tid < 3) a.part[b * kParts + kPartCount + tid] = s_cnt[tid];
+                if (!grid_barrier(st, phase)) return;
             }
         }
-        {
-            int mc = 0, ms = 0;
-            for (int s = s0 + tid; s < s1; s += kRefThreads) {
-                int off = 0, nc = 0, ns = 0;
-#pragma unroll
-                for (int d = 0; d < 8; ++d) {
-                    const int c = a.ncnt[8 * s + d];
-                    a.offs[8 * s + d] = off;
-                    off += c;
-                    nc += c > 0;
-                    ns += (c > a.ppn && child_may_split);
-                }
-                a.nch[s] = nc;
-                a.nsp[s] = ns;
-                mc += nc;
-                ms += ns;
-            }
-            mc = block_sum(mc, sh);
-            ms = block_sum(ms, sh);
-            if (tid == 0) {
-                a.part[b * kParts + 9] = mc;
-                a.part[b * kParts + 10] = ms;
-            }
-        }
-        if (!grid_barrier(st)) return;
+        resume = false;
 
         // ---- E: children and the scatter
-        int NC, NS;
-        {
-            int cbefore, sbefore;
-            parts_sums(a.part, 9, &cbefore, &NC, sh);
-            parts_sums(a.part, 10, &sbefore, &NS, sh);
-            if (total + NC > a.cap) {
-                status = kRefGrow;
-                need = NC;
-                break;
-            }
-            if (NS > a.smax) {
-                status = kRefOverflow;
-                break;
-            }
-            int cc = cbefore, sc = sbefore;
-            for (int base = s0; base < s1; base += kRefThreads) {
-                const int s = base + tid;
-                const int nc = s < s1 ? a.nch[s] : 0, ns = s < s1 ? a.nsp[s] : 0;
-                int tc, ts;
-                const int exc = block_excl(nc, &tc, sh);
-                const int exs = block_excl(ns, &ts, sh);
-                if (s < s1) {
-                    const int g = sp[s];
-                    const uint64_t k = a.key[g];
-                    const int cb = static_cast<int>(total) + cc + exc;
-                    int r = 0, rs = sc + exs;
-                    for (int d = 0; d < 8; ++d) {
-                        const int c = a.ncnt[8 * s + d];
-                        if (!c) continue;
-                        const int h = cb + r++;
-                        a.key[h] = (k << 3) | uint64_t(d);
-                        a.pbeg[h] = a.pbeg[g] + a.offs[8 * s + d];
-                        a.pend[h] = a.pbeg[h] + c;
-                        a.parent[h] = g;
-                        a.child_beg[h] = -1;
-                        a.nchild[h] = 0;
-                        if (c > a.ppn && child_may_split) spn[rs++] = h;
+        int before[3], all[3];
+        parts_sums<3>(a.part, kPartCount, before, all, sh6);
+        const int NC = all[0], NS = all[1], NT = all[2];
+        if (total + NC > a.cap) {
+            status = kRefGrow;
+            need = NC;
+            break;
+        }
+        if (NS > a.smax || NT > a.tmax) {
+            status = kRefOverflow;
+            break;
+        }
+        for (int base = s0; base < s1; base += kRefThreads) {
+            const int s = base + tid;
+            const int v = s < s1 ? a.nst[s] : 0, nt = s < s1 ? a.ntl[s] : 0;
+            int tv, tt;                                   // at most 8 x 256 children: 16 bits each
+            const int exv = block_excl(v, &tv, sh);
+            const int ext = block_excl(nt, &tt, sh);
+            if (s < s1) {
+                const int g = sp[s];
+                const uint64_t k = a.key[g];
+                const int pb = a.pbeg[g];
+                const int cb = static_cast<int>(total) + before[0] + (exv & 0xffff);
+                int r = 0, rs = before[1] + (exv >> 16), rt = before[2] + ext, off = pb, mask = 0;
+#pragma unroll
+                for (int d = 0; d < 8; ++d) {
+                    const int c = ncnt[8 * s + d];
+                    if (!c) continue;
+                    const int h = cb + r++;
+                    mask |= 1 << d;
+                    a.key[h] = (k << 3) | uint64_t(d);
+                    a.pbeg[h] = off;
+                    off += c;
+                    a.pend[h] = off;
+                    a.parent[h] = g;
+                    a.child_beg[h] = -1;
+                    a.nchild[h] = 0;
+                    a.cmask[h] = 0;
+                    if (c > a.ppn && child_may_split) {
+                        spn[rs] = h;
+                        tile_next[rs] = rt;
+                        rt += (c + tile - 1) / tile;
+                        if (NT != NS) {
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) ncnt_next[8 * rs + j] = 0;
+                        }
+                        ++rs;
                     }
-                    a.child_beg[g] = cb;
-                    a.nchild[g] = r;
                 }
-                cc += tc;
-                sc += ts;
+                a.child_beg[g] = cb;
+                a.nchild[g] = r;
+                a.cmask[g] = mask;
             }
+            before[0] += tv & 0xffff;
+            before[1] += tv >> 16;
+            before[2] += tt;
         }
         {
             int s = -1;
             for (int t = t0 + warp; t < t1; t += kRefWarps) {
-                s = seg_of(a.tile_off, S, t, s);
+                s = flat ? t : seg_of(tile_off, S, t, s);
                 const int g = sp[s];
-                const int f = a.tile_off[s];
-                const int pb = a.pbeg[g] + (t - f) * kWTile;
-                const int pe = min(a.pend[g], pb + kWTile);
-                int pos_d = 0, split_d = 0;                   // lane d < 8: next slot of digit d
+                const int f = flat ? t : tile_off[s];
+                const int pb = a.pbeg[g] + (t - f) * tile;
+                const int pe = min(a.pend[g], pb + tile);
+                int pos_d = 0, split_d = 0;               // lane d < 8: next slot of digit d
                 if (lane < 8) {
-                    pos_d = a.pbeg[g] + a.offs[8 * s + lane] + (a.pre[int64_t(lane) * T + t] - a.pre[int64_t(lane) * T + f]);
-                    split_d = a.ncnt[8 * s + lane] > a.ppn && child_may_split;
+                    pos_d = a.pbeg[g] + a.offs[8 * s + lane];
+                    if (!flat) pos_d += a.pre[int64_t(lane) * T + t] - a.pre[int64_t(lane) * T + f];
+                    split_d = ncnt[8 * s + lane] > a.ppn && child_may_split;
                 }
                 const unsigned splits = __ballot_sync(0xffffffffu, split_d);
-                for (int i0 = pb; i0 < pe; i0 += 128) {
-                    uint64_t kk[4];
-                    int oo[4];
+                for (int i0 = pb; i0 < pe; i0 += 256) {
+                    uint64_t kk[8];
+                    int oo[8];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
+                    for (int u = 0; u < 8; ++u) {
                         const int i = i0 + 32 * u + lane;
                         kk[u] = i < pe ? kin[i] : 0;
                         oo[u] = i < pe ? oin[i] : 0;
                     }
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
+                    for (int u = 0; u < 8; ++u) {
                         const bool valid = i0 + 32 * u + lane < pe;
-                        const int dg = valid ? static_cast<int>((kk[u] >> shift) & 7) : 8;
-                        const unsigned peers = __match_any_sync(0xffffffffu, dg);
-                        const int pos = __shfl_sync(0xffffffffu, pos_d, dg & 7) + __popc(peers & lt);
+                        const int dg = static_cast<int>((kk[u] >> shift) & 7);
+                        const unsigned b0 = __ballot_sync(0xffffffffu, dg & 1);
+                        const unsigned b1 = __ballot_sync(0xffffffffu, dg & 2);
+                        const unsigned b2 = __ballot_sync(0xffffffffu, dg & 4);
+                        const unsigned v = __ballot_sync(0xffffffffu, valid);
+                        const int pos = __shfl_sync(0xffffffffu, pos_d, dg) + __popc(octant_lanes(dg, b0, b1, b2, v) & lt);
                         if (valid) {
                             if ((splits >> dg) & 1u) {
                                 kout[pos] = kk[u];
@@ -1031,21 +1086,18 @@ __global__ void __launch_bounds__(kRefThreads) k_refine(RefineArgs a)
                                 a.final_ord[pos] = oo[u];
                             }
                         }
-#pragma unroll
-                        for (int d = 0; d < 8; ++d) {
-                            const unsigned m = __ballot_sync(0xffffffffu, dg == d);
-                            if (lane == d) pos_d += __popc(m);
-                        }
+                        if (lane < 8) pos_d += __popc(octant_lanes(lane, b0, b1, b2, v));
                     }
                 }
             }
         }
         if (b == 0 && tid == 0) st->lvl_off[level + 2] = total + NC;
-        if (!grid_barrier(st)) return;
-        lo = total;
+        if (!grid_barrier(st, phase)) return;
         total += NC;
         ++level;
+        Sprev = S;
         S = NS;
+        T = NT;
         cur ^= 1;
     }
 
@@ -1056,11 +1108,11 @@ __global__ void __launch_bounds__(kRefThreads) k_refine(RefineArgs a)
             int mine = 0;
             for (int64_t g = n0 + tid; g < n1; g += kRefThreads) mine += a.nchild[g] == 0;
             const int tot = block_sum(mine, sh);
-            if (tid == 0) a.part[b * kParts + 11] = tot;
+            if (tid == 0) a.part[b * kParts + kPartLeaf] = tot;
         }
-        if (!grid_barrier(st)) return;
+        if (!grid_barrier(st, phase)) return;
         int before, nleaves;
-        parts_sums(a.part, 11, &before, &nleaves, sh);
+        parts_sums<1>(a.part, kPartLeaf, &before, &nleaves, sh6);
         if (tid <= level + 1) s_lvl[tid] = reinterpret_cast<volatile long long*>(st->lvl_off)[tid];
         __syncthreads();
         int carry = before;
@@ -1083,6 +1135,7 @@ __global__ void __launch_bounds__(kRefThreads) k_refine(RefineArgs a)
         st->status = status;
         st->level = level;
         st->S = S;
+        st->T = T;
         st->cur = cur;
         st->need = need;
         st->total = total;
@@ -1117,6 +1170,8 @@ void read_two(const T* d0, const T* d1, T& v0, T& v1, cudaStream_t s)
     SFMM_CUDA(cudaStreamSynchronize(s));
 }
 
+int refine_tile(int64_t n) { return n < kTileLargeFrom ? kTileSmall : kTileLarge; }
+
 // The single-launch refinement unless SFMM_TREE_REFINE=levels asks for the
 // level-by-level launches (the tests run both), the device cannot launch
 // cooperatively, or the tile table would not fit 32-bit counts.
@@ -1128,7 +1183,7 @@ bool single_launch_refinement(int64_t n, int ppn)
     SFMM_CUDA(cudaGetDevice(&dev));
     SFMM_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
     const int64_t smax = std::max<int64_t>(1, n / (int64_t(ppn) + 1));
-    return coop && 8 * (n / kWTile + smax + 1) < (int64_t(1) << 31);
+    return coop && 8 * (n / refine_tile(n) + smax + 1) < (int64_t(1) << 31);
 }
 
 }  // namespace
@@ -1250,24 +1305,26 @@ void build_tree(Tree& t, const double* xyz, int max_level, int max_ppn, int vert
     if (single) {
         // one cooperative launch: all levels, the colleague lists, the leaves
         const int64_t smax = std::max<int64_t>(1, n / (int64_t(max_ppn) + 1));
-        const int64_t tmax = n / kWTile + smax + 1;
+        const int tile = refine_tile(n);
+        const int64_t tmax = n / tile + smax + 1;
         int dev = 0, sms = 0, occ = 0;
         SFMM_CUDA(cudaGetDevice(&dev));
         SFMM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         SFMM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_refine, kRefThreads, 0));
         SFMM_REQUIRE(occ > 0, FMM_ERR_UNSUPPORTED, "the refinement kernel cannot be resident");
-        // two root tiles per block, at least 32 blocks (small trees: the colleague
-        // and list steps are chains of dependent loads, one warp per node)
-        const int G = static_cast<int>(std::min<int64_t>(int64_t(occ) * sms, std::max<int64_t>(32, (n + 2 * kWTile - 1) / (2 * kWTile))));
-        DevBuf<int32_t> sp0, sp1, tile_off, hist, pre, ncnt, offs, nch, nsp, part;
+        // 2048 points per block (a small tile per warp), at least 32 blocks (small
+        // trees: chains of dependent loads, a warp per splitting node)
+        const int G = static_cast<int>(std::min<int64_t>(int64_t(occ) * sms, std::max<int64_t>(32, (n + 2047) / 2048)));
+        DevBuf<int32_t> sp0, sp1, tile_off, hist, pre, ncnt, offs, nst, ntl, cmask, part;
         DevBuf<RefineState> dst;
         sp0.alloc(smax, st);
         sp1.alloc(smax, st);
-        tile_off.alloc(smax, st);
-        ncnt.alloc(8 * smax, st);
+        tile_off.alloc(2 * smax, st);
+        ncnt.alloc(16 * smax, st);
         offs.alloc(8 * smax, st);
-        nch.alloc(smax, st);
-        nsp.alloc(smax, st);
+        nst.alloc(smax, st);
+        ntl.alloc(smax, st);
+        cmask.alloc(cap, st);
         hist.alloc(8 * tmax, st);
         pre.alloc(8 * tmax, st);
         part.alloc(size_t(kParts) * G, st);
@@ -1275,6 +1332,8 @@ void build_tree(Tree& t, const double* xyz, int max_level, int max_ppn, int vert
         if (S) {
             const int32_t z = 0;
             SFMM_CUDA(cudaMemcpyAsync(sp0.ptr, &z, 4, cudaMemcpyHostToDevice, st));
+            SFMM_CUDA(cudaMemsetAsync(tile_off.ptr, 0, 4, st));
+            SFMM_CUDA(cudaMemsetAsync(ncnt.ptr, 0, 32, st));
         }
         t.colleague.alloc(27 * cap, st);
         t.leaf_id.alloc(cap, st);
@@ -1285,6 +1344,7 @@ void build_tree(Tree& t, const double* xyz, int max_level, int max_ppn, int vert
         const int stall_test = stall_env && std::strcmp(stall_env, "1") == 0;
         RefineState h{};
         h.S = S;
+        h.T = S ? static_cast<int>((n + tile - 1) / tile) : 0;
         h.total = 1;
         h.lvl_off[1] = 1;
         for (;;) {
@@ -1306,13 +1366,17 @@ void build_tree(Tree& t, const double* xyz, int max_level, int max_ppn, int vert
             ra.final_ord = t.order.ptr;
             ra.sp[0] = sp0.ptr;
             ra.sp[1] = sp1.ptr;
-            ra.tile_off = tile_off.ptr;
+            ra.tile_off[0] = tile_off.ptr;
+            ra.tile_off[1] = tile_off.ptr + smax;
+            ra.ncnt[0] = ncnt.ptr;
+            ra.ncnt[1] = ncnt.ptr + 8 * smax;
             ra.hist = hist.ptr;
             ra.pre = pre.ptr;
-            ra.ncnt = ncnt.ptr;
             ra.offs = offs.ptr;
-            ra.nch = nch.ptr;
-            ra.nsp = nsp.ptr;
+            ra.nst = nst.ptr;
+            ra.ntl = ntl.ptr;
+            ra.cmask = cmask.ptr;
+            ra.tile = tile;
             ra.part = part.ptr;
             ra.smax = static_cast<int>(smax);
             ra.tmax = static_cast<int>(tmax);
@@ -1335,7 +1399,10 @@ void build_tree(Tree& t, const double* xyz, int max_level, int max_ppn, int vert
                 t.colleague.grow(27 * cap, 27 * keep, st);
                 t.leaf_id.alloc(cap, st);
                 t.leaf_node.alloc(cap, st);
+                cmask.grow(cap, keep, st);
                 h.status = kRefDone;
+                h.resume = 1;
+                h.bar_count = 0;
                 continue;
             }
             SFMM_REQUIRE(h.status == kRefDone, FMM_ERR_UNSUPPORTED, "tree refinement: work exceeded its bounds");
