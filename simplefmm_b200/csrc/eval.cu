@@ -52,82 +52,144 @@ __global__ void k_gather_q(const double* __restrict__ Q, const int32_t* __restri
 }
 
 // P2M (fmm.hpp:524-556): warp per leaf of level >= 2, lanes over points.
-// The lanes' terms q_b S_n^m go through a per-warp staging block of
-// kP2MStage values: each lane writes its terms, then two lanes per value add
-// the 32 lanes' entries (16 each and one shuffle) into the coefficient.  That
-// is about four instructions per term and lane, against a five-step warp sum.
-constexpr int kP2MStage = 16;                   // values staged per reduction
-constexpr int kP2MLd = 33;                      // doubles per staged value (32 lanes + pad)
-constexpr size_t kP2MStageBytes = size_t(kP2MStage) * kP2MLd * sizeof(double) + kP2MStage * sizeof(int);
 
-template<int QD>
-__global__ void __launch_bounds__(kMaxWarps * 32) k_p2m(EvalArgs a)
+// P2M: lanes over azimuthal orders.
+// S_n^m = P_n^m(z, r^2) d_m with d_m = (-x + iy)^m times a constant and P real,
+// so a lane that holds one m needs one complex power a point and then a real
+// three-term recurrence, and its sums over the points stay in its registers.
+// A lane takes the orders m = i and m = p - i (p + 2 terms together, the same
+// for every lane), a point takes L = p / 2 + 1 lanes, and a warp 32 / L points
+// at a time (5 at p = 10).  A warp takes a few leaves: the coefficients by step
+// are tabled once a block.
+//
+// Measured against a lane per point (complex recurrence, every term staged in
+// shared memory and summed over the lanes, rounds of 32 points half empty at
+// 10 to 30 points a leaf): p = 10, 300k points 78 -> 60 us, 1M 223 -> 170; p = 12,
+// 16M points 2.82 -> 2.18 ms.  Two points a lane for more independent chains took
+// 128 registers and was slower (1M 201 us).
+__host__ __device__ constexpr int lanes_per_point(int p) { return p / 2 + 1; }
+
+// Step j of lane i: (n, m); false for the middle order's unused second half.
+__device__ __forceinline__ bool slot_nm(int p, int i, int j, int& n, int& m)
 {
+    const bool second = j > p - i;
+    m = second ? p - i : i;
+    n = second ? j - 1 : i + j;               // (p - i) + (j - (p - i + 1))
+    return !(second && 2 * i == p);
+}
+
+// Recurrence coefficients by step and lane, {z, r^2}; 0 where an order starts
+// (the lane then restarts P at 1).
+__device__ __forceinline__ void fill_steps(int p, int L, double2* coef)
+{
+    for (int t = threadIdx.x; t < (p + 2) * L; t += blockDim.x) {
+        int n, m;
+        const bool on = slot_nm(p, t % L, t / L, n, m);
+        double2 c{0.0, 0.0};
+        if (on && n == m + 1) c.x = c_harm.sub[m];
+        if (on && n > m + 1) c = double2{c_harm.ra[tri(n, m)], c_harm.rb[tri(n, m)]};
+        coef[t] = c;
+    }
+}
+
+// d_i and d_{p-i} of the lane's point: d_i by squarings, d_{p-i} from the
+// lanes of the same point that hold i' = L - 1 - i and i' = L - 1.
+__device__ __forceinline__ void lane_powers(int p, int L, int lane, int i, double x, double y, double n1, double n2, cplx& d1,
+                                            cplx& d2)
+{
+    const cplx b{-x, y};
+    cplx q = b;
+    d1 = (i & 1) ? b : cplx{1.0, 0.0};
+#pragma unroll
+    for (int k = 1; k < 4; ++k) {
+        if ((L - 1) >> k == 0) break;
+        q = cplx{q.re * q.re - q.im * q.im, 2.0 * q.re * q.im};
+        const cplx v = cmul(d1, q);
+        if ((i >> k) & 1) d1 = v;
+    }
+    const int first = lane - i, other = (first + L - 1 - i) & 31, top = (first + L - 1) & 31;
+    const cplx t{__shfl_sync(0xffffffffu, d1.re, top), __shfl_sync(0xffffffffu, d1.im, top)};
+    const cplx o{__shfl_sync(0xffffffffu, d1.re, other), __shfl_sync(0xffffffffu, d1.im, other)};
+    d2 = cmul(t, o);
+    if (p & 1) d2 = cmul(d2, b);
+    d1 = cplx{n1 * d1.re, n1 * d1.im};
+    d2 = cplx{n2 * d2.re, n2 * d2.im};
+}
+
+constexpr int kLeafWarps = 4;
+
+template<int P>
+constexpr size_t p2m_smem()
+{
+    return sizeof(double2) * (P + 2) * lanes_per_point(P) + sizeof(cplx) * kLeafWarps * (P + 2) * 32;
+}
+
+// P2M: warp per leaf of level >= 2, all charge components in turn.
+template<int P>
+__global__ void __launch_bounds__(kLeafWarps * 32, P <= 8 ? 6 : P <= 12 ? 5 : 4) k_p2m(EvalArgs a)
+{
+    constexpr int L = lanes_per_point(P), GR = 32 / L, NJ = P + 2;
     extern __shared__ double smem[];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    const size_t per_warp = size_t(a.qdim) * a.T * sizeof(cplx) + kP2MStageBytes;
-    char* wbase = reinterpret_cast<char*>(smem) + w * per_warp;
-    cplx* acc = reinterpret_cast<cplx*>(wbase);
-    double* accd = reinterpret_cast<double*>(wbase);
-    double* stage = reinterpret_cast<double*>(wbase + size_t(a.qdim) * a.T * sizeof(cplx));
-    int* sidx = reinterpret_cast<int*>(stage + kP2MStage * kP2MLd);
-    const int j = lane & 15, h = lane >> 4;
+    double2* coef = reinterpret_cast<double2*>(smem);
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    cplx* stage = reinterpret_cast<cplx*>(coef + NJ * L) + w * NJ * 32;
+    const int grp = lane / L, i = lane - grp * L;
+    const double n1 = c_harm.dprod[i], n2 = c_harm.dprod[P - i];
+    fill_steps(P, L, coef);
+    __syncthreads();
     const int64_t nfar = a.n_leaves - a.far_leaf0;
-    for (int64_t f = blockIdx.x * int64_t(nw) + w; f < nfar; f += int64_t(gridDim.x) * nw) {
-        const int g = a.leaf_node[a.far_leaf0 + f];
+    for (int64_t f = blockIdx.x * int64_t(kLeafWarps) + w; f < nfar; f += int64_t(gridDim.x) * kLeafWarps) {
+        const int64_t g = a.leaf_node[a.far_leaf0 + f];
         if (a.own_leaf && !a.own_leaf[a.far_leaf0 + f]) {      // another shard's leaf: zero moments
-            for (int t = lane; t < a.qdim * a.T; t += 32) a.M[int64_t(g) * a.qdim * a.T + t] = cplx{0, 0};
+            for (int t = lane; t < a.qdim * a.T; t += 32) a.M[g * a.qdim * a.T + t] = cplx{0, 0};
             continue;
         }
         const int l = level_of(a, g);
         double c[3];
         node_center(*a.box, a.key[g], l, c);
-        for (int t = lane; t < a.qdim * a.T; t += 32) acc[t] = cplx{0, 0};
-        __syncwarp();
         const int b0 = a.pbeg[g], b1 = a.pend[g];
-        for (int base = b0; base < b1; base += 32) {
-            const int i = base + lane;
-            const bool on = i < b1;
-            const double x = on ? a.fx[i] - c[0] : 0, y = on ? a.fy[i] - c[1] : 0, z = on ? a.fz[i] - c[2] : 0;
-            double q[QD];                                 // QD = qdim: the charges stay in registers
+        for (int b = 0; b < a.qdim; ++b) {
+            cplx acc[NJ];
 #pragma unroll
-            for (int b = 0; b < QD; ++b) q[b] = on ? a.qs[b * a.n + i] : 0.0;
-            int cnt = 0;                                  // staged values (the same in every lane)
-            auto flush = [&](int nv) {
-                __syncwarp();
-                double sum = 0.0;
-                if (j < nv) {
-                    const double* col = stage + j * kP2MLd + h * 16;
+            for (int j = 0; j < NJ; ++j) acc[j] = cplx{0, 0};
+            for (int base = b0; base < b1; base += GR) {
+                const int k = base + grp;
+                const bool on = grp < GR && k < b1;
+                const double x = on ? a.fx[k] - c[0] : 0, y = on ? a.fy[k] - c[1] : 0, z = on ? a.fz[k] - c[2] : 0;
+                const double q = on ? a.qs[int64_t(b) * a.n + k] : 0.0, r2 = x * x + y * y + z * z;
+                double p1 = 0.0, p2 = 0.0;
+                cplx d, d2;
+                lane_powers(P, L, lane, i, x, y, q * n1, q * n2, d, d2);
 #pragma unroll
-                    for (int u = 0; u < 16; ++u) sum += col[u];
+                for (int j = 0; j < NJ; ++j) {
+                    const double2 cf = coef[j * L + i];
+                    const double v = cf.x * z * p1 - cf.y * r2 * p2;
+                    const bool second = j > 0 && j == P - i + 1;
+                    p2 = p1;
+                    p1 = j == 0 || second ? 1.0 : v;
+                    if (second) d = d2;
+                    acc[j].re += d.re * p1;
+                    acc[j].im += d.im * p1;
                 }
-                sum += __shfl_xor_sync(0xffffffffu, sum, 16);
-                if (h == 0 && j < nv) accd[sidx[j]] += sum;
-                __syncwarp();
-            };
-            for_each_harmonic(a.p, x, y, z, c_harm, [&](int n, int m, cplx s) {
-                const int t = tri(n, m);
+            }
 #pragma unroll
-                for (int b = 0; b < QD; ++b) {
-                    stage[cnt * kP2MLd + lane] = q[b] * s.re;
-                    stage[(cnt + 1) * kP2MLd + lane] = q[b] * s.im;
-                    if (lane == 0) {
-                        sidx[cnt] = 2 * (b * a.T + t);
-                        sidx[cnt + 1] = 2 * (b * a.T + t) + 1;
-                    }
-                    cnt += 2;
-                    if (cnt == kP2MStage) {
-                        flush(kP2MStage);
-                        cnt = 0;
-                    }
+            for (int j = 0; j < NJ; ++j) stage[j * 32 + lane] = acc[j];
+            __syncwarp();
+            cplx* M = a.M + (g * a.qdim + b) * a.T;
+            for (int t = lane; t < NJ * L; t += 32) {
+                const int j = t / L, k = t - j * L;
+                int n, m;
+                if (!slot_nm(P, k, j, n, m)) continue;
+                cplx s = stage[j * 32 + k];
+#pragma unroll
+                for (int r = 1; r < GR; ++r) {
+                    s.re += stage[j * 32 + r * L + k].re;
+                    s.im += stage[j * 32 + r * L + k].im;
                 }
-            });
-            if (cnt) flush(cnt);
+                M[tri(n, m)] = s;
+            }
+            __syncwarp();
         }
-        __syncwarp();
-        cplx* M = a.M + int64_t(g) * a.qdim * a.T;
-        for (int t = lane; t < a.qdim * a.T; t += 32) M[t] = acc[t];
-        __syncwarp();
     }
 }
 
@@ -312,25 +374,27 @@ void allow_smem(KernelT k, size_t smem)
     allow_max_smem(k);
 }
 
-// P2M for one, two or three charge components
-void launch_p2m(const EvalArgs& a, int64_t nfar, int w, size_t smem, cudaStream_t st)
+template<int P>
+void launch_p2m_p(const EvalArgs& a, int64_t nfar, cudaStream_t st)
 {
-    switch (a.qdim) {
-    case 1:
-        allow_smem(k_p2m<1>, smem);
-        k_p2m<1><<<blocks_for(nfar, w, 65535), w * 32, smem, st>>>(a);
-        break;
-    case 2:
-        allow_smem(k_p2m<2>, smem);
-        k_p2m<2><<<blocks_for(nfar, w, 65535), w * 32, smem, st>>>(a);
-        break;
-    case 3:
-        allow_smem(k_p2m<3>, smem);
-        k_p2m<3><<<blocks_for(nfar, w, 65535), w * 32, smem, st>>>(a);
-        break;
-    default: SFMM_REQUIRE(false, FMM_ERR_UNSUPPORTED, "P2M: charges have 1, 2 or 3 components");
+    allow_smem(k_p2m<P>, p2m_smem<P>());
+    int nb = 0, dev = 0, sms = 0;
+    SFMM_CUDA(cudaGetDevice(&dev));
+    SFMM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    SFMM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_p2m<P>, kLeafWarps * 32, p2m_smem<P>()));
+    k_p2m<P><<<blocks_for(nfar, kLeafWarps, 4 * std::max(1, nb) * sms), kLeafWarps * 32, p2m_smem<P>(), st>>>(a);
+}
+
+// P2M by expansion order (the sums are registers, one per step)
+template<int P = 0>
+void launch_p2m(const EvalArgs& a, int64_t nfar, cudaStream_t st)
+{
+    if (a.p == P) {
+        launch_p2m_p<P>(a, nfar, st);
+        SFMM_CHECK_LAUNCH();
+    } else if constexpr (P < kMaxOrder) {
+        launch_p2m<P + 1>(a, nfar, st);
     }
-    SFMM_CHECK_LAUNCH();
 }
 
 template<int KM>
@@ -641,9 +705,7 @@ void plan_evaluate(Plan& pl, const double* Q, double* pot, double* field, cudaEv
     const bool far = t.depth >= 2;
     if (far) {
         const int64_t nfar = t.n_leaves - a.far_leaf0;
-        const size_t sm_p2m_w = size_t(qd) * T * sizeof(cplx) + kP2MStageBytes;
-        const int w_p2m = warps_for(0, sm_p2m_w);
-        launch_p2m(a, nfar, w_p2m, sm_p2m_w * w_p2m, st);
+        launch_p2m(a, nfar, st);
         const size_t head = (32 + 2 * 4 * (2 * kMaxOrder + 1)) * sizeof(double);
         const size_t sm_m2m_w = 2 * size_t(qd) * T * sizeof(cplx);
         const int w_m2m = warps_for(head, sm_m2m_w);
@@ -764,9 +826,7 @@ void plan_evaluate_stage(Plan& pl, const double* Q, double* pot, double* field, 
         launch_p2p(a, sms, side);
         SFMM_CUDA(cudaEventRecord(pl.join, side));
         if (far) {
-            const size_t sm_p2m_w = size_t(qd) * T * sizeof(cplx) + kP2MStageBytes;
-            const int w_p2m = warps_for(0, sm_p2m_w);
-            launch_p2m(a, nfar, w_p2m, sm_p2m_w * w_p2m, st);
+            launch_p2m(a, nfar, st);
         }
         return;
     }

@@ -68,6 +68,7 @@ SFMM_HD uint32_t compact3(uint64_t x)
 struct HarmCoef {
     double diag[kMaxOrder + 1];
     double sub[kMaxOrder + 1];
+    double dprod[kMaxOrder + 1];         // diag[1] .. diag[m] multiplied
     double ra[kMaxTri];
     double rb[kMaxTri];
     signed char tn[kMaxTri];             // tri index -> n
@@ -79,6 +80,7 @@ inline void fill_harm_coef(HarmCoef& h)
     for (int m = 0; m <= kMaxOrder; ++m) {
         h.diag[m] = m == 0 ? 1.0 : std::sqrt((2.0 * m - 1) / (2.0 * m));
         h.sub[m] = std::sqrt(2.0 * m + 1);
+        h.dprod[m] = m == 0 ? 1.0 : h.dprod[m - 1] * h.diag[m];
     }
     for (int n = 0; n <= kMaxOrder; ++n)
         for (int m = 0; m <= n; ++m) {
