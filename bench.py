@@ -70,11 +70,21 @@ def m2l_useful_flops(p: int) -> int:
 
 
 def m2l_mma_flops(p: int) -> int:
-    """FP64 tensor-core operations the M2L kernel (k_m2l_mma) issues per
-    ilist pair: its compile-time MMA schedule for one 8-column tile (8x8x4
-    DMMA, 512 flops each, zero-padded operator fragments) over 8 columns."""
+    """FP64 tensor-core operations the M2L kernel issues per ilist pair and
+    column (8x8x4 DMMA, 512 flops over 8 columns, zero-padded operator
+    fragments).  p = 2..12, k_m2l_tile: the fragments of one offset (rotation
+    of orders < p, z-translation of re and im, inverse rotation, the order-p
+    sources' map); columns without a source at an offset come on top.
+    Above, k_m2l_mma: its schedule for one 8-column tile."""
     rt = lambda n: (n + 8) // 8  # noqa: E731
     kc = lambda n: (n + 4) // 4  # noqa: E731
+    up = lambda a, b: -(-a // b)  # noqa: E731
+    if 2 <= p <= 12:
+        rot = sum(2 * rt(n) * kc(n) for n in range(p))
+        tz = sum(up(p + 2 - k, 8) * up(p - k, 4) for k in range(p))
+        inv = sum(rt(j) * (up(min(j, p - 1) + 1, 4) + up(min(j, p - 1), 4)) for j in range(p + 2))
+        top = 2 * up((p + 1) * (p + 2) // 2, 8) * up(p + 1, 4)
+        return (rot + 2 * tz + inv + top) * 512 // 8
     rot = sum(2 * rt(n) * kc(n) for n in range(p + 1))
     tz = sum(((p + 2 - k + 7) // 8) * 2 * ((p - k + 3) // 4 if k < p else 0) for k in range(p + 2))
     inv = sum(rt(j) * kc(j) * 2 * (1 if j == p + 1 else 2) for j in range(p + 2))
@@ -189,12 +199,24 @@ def int8_peak_tops(torch) -> float:
     return best
 
 
+def m2l_i8_phases(p: int) -> list[tuple[int, int]]:
+    """(operator rows, moments) of the dense products of the mixed plans' M2L
+    (k_m2l_i8).  From p = 7 on the field local's (p+2)^2 rows over the source
+    orders < p serve the potential local too, which adds order p alone;
+    below, both locals' rows run over all orders (the field local's entries of
+    order p are zero)."""
+    if p >= 7:
+        return [((p + 2) ** 2, p ** 2), ((p + 1) ** 2, 2 * p + 1)]
+    return [((p + 1) ** 2 + (p + 2) ** 2, (p + 1) ** 2)]
+
+
 def m2l_i8_ops(p: int) -> int:
     """int8 tensor-core operations of the mixed plans' M2L (k_m2l_i8) per
     ilist pair and charge component, on the nonzero entries of its dense
-    operator: potential-local rows (p+1)^2 x (p+1)^2 moments, field-local
-    rows (p+2)^2 x p^2, each a product of four-digit numbers taken as ten
-    8-bit digit products (2 ops per multiply-add)."""
+    operators, each a product of four-digit numbers taken as ten 8-bit digit
+    products (2 ops per multiply-add)."""
+    if p >= 7:
+        return 2 * 10 * sum(r * k for r, k in m2l_i8_phases(p))
     return 2 * 10 * ((p + 1) ** 4 + (p + 2) ** 2 * p ** 2)
 
 
@@ -256,11 +278,8 @@ def roofline_i8(torch, pairs: int, p: int, m2l_ms: float, m2l_bytes: int) -> dic
     ops = pairs * m2l_i8_ops(p)
     achieved = ops / (m2l_ms * 1e-3) / 1e12
     peak = int8_peak_tops(torch)
-    rows, k = (p + 1) ** 2 + (p + 2) ** 2, (p + 1) ** 2
-    # what the instruction shape allows: N = 128 of the 256 an MMA costs the
-    # same for (four int32 accumulators fill tensor memory), rows padded to
-    # 128, K to 32
-    shape = 0.5 * rows / (128 * -(-rows // 128)) * k / (32 * -(-k // 32))
+    # what the instruction shape allows: rows padded to 128, K to 32
+    shape = m2l_i8_ops(p) / (20 * sum(128 * -(-r // 128) * 32 * -(-k // 32) for r, k in m2l_i8_phases(p)))
     return {"bound": "tensor", "pipe": "int8 tensor cores (tcgen05.mma kind::i8, M=128 N=128 K=32)", "kernel": "k_m2l_i8",
             "achieved": achieved, "peak": peak, "unit": "TOPS", "frac": achieved / peak,
             "peak_source": "int8 GEMM (torch._int_mm 8192^3, cuBLASLt) measured in this run; MEASURED_PEAKS.json "
@@ -731,7 +750,8 @@ def main():
             "tree_build_phases": dict(build, peak_hbm_gbs=hbm, peak_source=peaks_src,
                                       work="algorithmic bytes of each phase (fmm_tree_build_phases) / its device time"),
             "roofline": roofline_i8(torch, pairs, p, m2l_avg, m2l_bytes) if tensor_i8 else {
-                         "bound": "tensor", "pipe": "FP64 tensor cores (DMMA 8x8x4)", "kernel": "k_m2l_mma",
+                         "bound": "tensor", "pipe": "FP64 tensor cores (DMMA 8x8x4)",
+                         "kernel": "k_m2l_tile" if 2 <= p <= 12 else "k_m2l_mma",
                          "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                          "peak_source": "FP64 DGEMM (torch float64 matmul 8192^3, cuBLAS DMMA) measured in this run; "
                                         "MEASURED_PEAKS.json has no FP64 figure",

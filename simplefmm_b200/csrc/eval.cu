@@ -51,9 +51,7 @@ __global__ void k_gather_q(const double* __restrict__ Q, const int32_t* __restri
     }
 }
 
-// P2M (fmm.hpp:524-556): warp per leaf of level >= 2, lanes over points.
-
-// P2M: lanes over azimuthal orders.
+// P2M (fmm.hpp:524-556): warp per leaf of level >= 2, lanes over azimuthal orders.
 // S_n^m = P_n^m(z, r^2) d_m with d_m = (-x + iy)^m times a constant and P real,
 // so a lane that holds one m needs one complex power a point and then a real
 // three-term recurrence, and its sums over the points stay in its registers.

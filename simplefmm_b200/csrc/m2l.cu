@@ -2,10 +2,13 @@
 // local (order p) and the field local (order p + 1, source orders <= p - 1)
 // produced from one rotation and one z-translation per pair.
 //
-// Kernels: k_m2l_mma (FP64 tensor cores, below) is the path for p >= 2;
-// k_m2l_tf32 the mixed-precision one for p >= 11; k_m2l_rows (this header)
-// runs p < 2 and any plan whose DMMA kernel does not fit the device, and a
-// plan created with SFMM_M2L_KERNEL=rows in the environment (a test switch).
+// Kernels: k_m2l_mma (FP64 tensor cores, below) takes p >= 13 and sparse lists
+// (m2l_sparse, fmm_internal.cuh: few sources per target, as on a shell, where
+// the tiled kernel of m2l_tile.cu, the path of p = 2..12, would run mostly empty
+// slots); k_m2l_tf32 is the mixed-precision one for p >= 11 where the int8
+// kernel does not apply; k_m2l_rows (this header) runs p < 2 and any plan whose
+// DMMA kernel does not fit the device, and a plan created with
+// SFMM_M2L_KERNEL=rows in the environment (a test switch).
 //
 // Work decomposition.  One block per sibling group: the children of one node
 // (<= 8 targets at level l >= 2).  Their interaction lists are contiguous and

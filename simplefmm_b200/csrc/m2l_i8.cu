@@ -57,7 +57,7 @@
 // whatever the MMAs.  Copies of whole 128-byte lines (eight lanes a row, into
 // the 128-byte swizzle), arrivals by the copies themselves, the proxy fence in
 // a thread of its own and two K steps per set of barrier waits brought a step
-// to 995 cycles (shared rows: 18 instead of 12 steps a slot), 19.3 ms, against
+// to 995 cycles (shared rows: 12 instead of 18 steps a slot), 19.3 ms, against
 // 640 cycles of MMA.  TMA gathers of the rows (tile::gather4) took 2450 cycles
 // a step.  1M Plummer points, p = 10: 7.1 -> 3.8 ms.
 //

@@ -4,38 +4,54 @@
 //
 // Work decomposition.  All targets of one octant (position in the parent) at
 // one level have their sources at the same offsets d, so for a given d they
-// share the whole operator: rotation class, distance and azimuth.  A tile is
-// up to 32 columns (16 above p = 10): the children in one octant of up to 32
-// consecutive split parents of a level (a column is a target and a charge
-// component).  A block runs over the tile's slots (the offsets that occur, at
-// most 189 of the 6 x 6 x 6 box around the target); a target without a source
-// in a slot takes zero moments.  Every operator fragment read serves 4 MMAs
-// and the sums of all slots stay on the SM.  Large trees order a level's
-// parents by which of their 27 neighbours are split, so that a tile's targets
-// have the same slots.
+// share the whole operator: rotation class, distance and azimuth.  A warp owns
+// 8 columns (the N of the MMA; a column is a target and a charge component):
+// children in one octant of consecutive split parents of a level.  The block's
+// warps run over the same slots (the offsets that occur, at most 189 of the
+// 6 x 6 x 6 box around the target) with one copy of the slot's operators; a
+// target without a source in a slot takes zero moments.  Large trees order a
+// level's parents by which of their 27 neighbours are split, so that a block's
+// targets have the same slots.
 //
 // Per slot, with expansions of the level scaled by the box size w
 // (M~_n = w^-n M_n, L_j = w^-(j+1) L~_j; the factor w^-n rides on the phases):
 //   R  X = e^{i m phi} M~ (formed as operands are read), W_n = (P_n Re X_n,
-//      Q_n Im X_n) for orders n < p; and D += the whole map of the order-p
-//      moments into the potential local's frame of this azimuth
-//   T  Lz^k = T_k W^k, the distance in the operator
-//   I  S_j += (PB_j Re Lz_j, QB_j Im Lz_j), orders j <= p + 1
-// The potential local (order p, sources <= p) and the field local (order
-// p + 1, sources < p) differ by the order-p sources alone, so S serves both
-// and D is the rest.  S and D accumulate in registers over the slots of one
-// azimuth (36 of up to 189) and are then turned by e^{-i m phi} into the tile's
-// sums in shared memory, each element by its one owner: no atomics, and a
-// target's result does not depend on its tile (absent sources add zeros).
+//      Q_n Im X_n) for orders n < p
+//   T  Lz^k = T_k W^k, the distance in the operator, in place
+//   I  L_j += e^{-i m phi} (PB_j Re Lz_j, QB_j Im Lz_j), orders j <= p + 1,
+//      in registers over the slots of a part
+// and after the slots a second pass D: the whole map (rotate, translate,
+// rotate back) of the order-p moments, which the potential local (order p,
+// sources <= p) has and the field local (order p + 1, sources < p) has not.
+// The rest serves both.
 //
-// A slot's operators (one class, 51 KB at p = 10) and the next slot's moments
-// come by bulk copies while the stages run; the moments, W and Lz change places
-// in two buffers.  Three barriers per slot of 32 columns.  Operand buffers are
-// laid out so that fragment loads and stores are free of bank conflicts.
+// A warp's operands are its own, so its stages need no block barrier; the
+// block shares only the operators.  These come by bulk copies, a buffer or two
+// per stage (D: a ring of four), each with a full and an empty mbarrier; one
+// warp per buffer refills it when every warp has left it.  All waits are
+// bounded.  Operand buffers are laid out so that fragment loads and stores are
+// free of bank conflicts.
+//
+// The sum over slots has a fixed association, whatever the block: six parts
+// (the planes of one y offset, 36 slots each), added in part order.  One block
+// runs all parts of its columns and adds each to LA / LB as it ends; or, for
+// levels too small to fill the GPU so (kTileSplitRows), a block runs one part
+// and k_tile_sum adds the parts in the same order.  No atomics.
+//
+// What bounds it: the FP64 unit, which DMMA (m8n8k4: 16 cycles a warp and
+// sub-partition, latency 26) shares with DFMA, and the shared-memory operand
+// reads between the MMAs; a slot of 8 warps takes about 14,000 cycles at
+// p = 10, of which the unit is busy 8,400.  Three designs on the way, 4M Plummer
+// points, p = 10: run-time job lists over 32 shared columns and three block
+// barriers a slot 57 ms; the chunk loops unrolled 49 ms; a warp's own 8 columns
+// 41 ms; loads moved before the stores they do not depend on and the ring for D
+// 36.9 ms; in-place T and one refilling warp per buffer 35.7 ms.  (Per-warp
+// straight-line code, 197 KB of it, missed the instruction cache: 114 ms.)
 //
 // Before (one block per sibling group, 8-column tiles of one class, an operator
-// fragment load per MMA, five barriers per 8 columns), 4M Plummer points,
-// p = 10: 69.6 ms, the FP64 tensor pipe 24% busy.
+// fragment load per MMA, five barriers per 8 columns: m2l.cu), 69.6 ms at that
+// size, the FP64 unit 24% busy; 300k points p = 10 5.69 -> 3.42 ms; 400k p = 6
+// potential 3.81 -> 2.21; 100k p = 8 1.19 -> 0.72; 2k p = 10 0.226 -> 0.185.
 #include <cub/device/device_radix_sort.cuh>
 
 #include <algorithm>
