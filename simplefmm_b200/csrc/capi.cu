@@ -473,6 +473,7 @@ int fmm_plan_capture(fmm_plan* plan, const double* Q, double* pot, double* field
     }
     SFMM_CUDA(cudaStreamEndCapture(c.stream, &pl.graph));
     SFMM_CUDA(cudaGraphInstantiate(&pl.graph_exec, pl.graph, 0));
+    pl.graph_i8 = pl.i8;
     API_CATCH
 }
 

@@ -766,9 +766,10 @@ void plan_set_shard(Plan& pl, int index, int count)
     if (count > 1) pl.i8.reset();                 // sharded mixed plans take the rotation M2L
     pl.own_parent_b.clear();
     pl.own_parent_e.clear();
+    // a mixed plan without its int8 data: the FP64 M2L's tiles, once
+    if (!pl.mt_on) m2l_tile_setup(pl);
     if (count == 1) {
         pl.own_leaf.release();
-        m2l_tile_setup(pl);
         return;
     }
     // this shard's leaves, level by level, balanced by points (shard_ranges.h)
@@ -794,7 +795,7 @@ void plan_set_shard(Plan& pl, int index, int count)
         pl.own_parent_b.push_back(b + shard_begin(nq, count, index));
         pl.own_parent_e.push_back(b + shard_end(nq, count, index));
     }
-    m2l_tile_setup(pl);
+    m2l_tile_shard(pl);
 }
 
 void plan_evaluate_stage(Plan& pl, const double* Q, double* pot, double* field, int stage)

@@ -148,10 +148,14 @@ struct Plan {
     DevBuf<int4> p2p_item;
     DevBuf<int32_t> p2p_row, p2p_parts, p2p_rowoff, p2p_ctr;
     DevBuf<int32_t> m2l_ctr;                  // M2L work counter (m2l.cu, m2l_tile.cu)
-    // tiled M2L (m2l_tile.cu): split parents by level, chunks of them, the blocks' slot tables
-    DevBuf<int32_t> mt_parent, mt_table;
-    DevBuf<int4> mt_chunk;
-    int64_t mt_chunks = 0;
+    // tiled M2L (m2l_tile.cu): the tiles of the whole tree and of this shard's
+    // parents (split parents by level, chunks of them), the blocks' slot tables
+    struct TileList {
+        DevBuf<int32_t> parent;
+        DevBuf<int4> chunk;
+        int64_t chunks = 0;
+    } mt_all, mt_shard;
+    DevBuf<int32_t> mt_table;
     int mt_tpb = 0, mt_warps = 0;
     bool mt_on = false;                       // the plan takes the tiled M2L (mt_groups' parents apart)
     bool mt_split = false;                    // the parts of a tile in blocks of their own
@@ -183,9 +187,12 @@ struct Plan {
     cudaEvent_t ev[8] = {};
     cudaEvent_t fork = nullptr, join = nullptr;   // side stream: start after the charges, join before the sums
     cudaEvent_t io_start = nullptr, io_done = nullptr;   // host-array evaluations: output copies on the copy stream
-    // one captured evaluation (fmm_plan_capture / fmm_plan_replay)
+    // one captured evaluation (fmm_plan_capture / fmm_plan_replay).  It runs on
+    // this plan's buffers, so a shard switch leaves those it uses alone: the
+    // whole tree's tiles (mt_all) stay, the int8 data is held here
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graph_exec = nullptr;
+    std::shared_ptr<I8PlanData> graph_i8;
 };
 
 void plan_init(Plan& pl);
@@ -196,8 +203,8 @@ void shift_setup(Plan& pl);
 void shift_m2m(Plan& pl, const EvalArgs& a, int lp, cudaStream_t st);
 void shift_l2l(Plan& pl, const EvalArgs& a, int lc, cudaStream_t st);
 // m2l_tile.cu: the FP64 M2L of orders kTileMinOrder..kTileMaxOrder; operators
-// per (device, p), set-up per plan (after shift_setup; again after
-// plan_set_shard), launch (false: the plan takes another kernel)
+// per (device, p), set-up per plan (after shift_setup), the tiles of a shard's
+// parents (plan_set_shard), launch (false: the plan takes another kernel)
 constexpr int kTileMinOrder = 2, kTileMaxOrder = 12;
 constexpr int kTf32MinOrder = 11;         // lowest order at which mixed plans use the TF32 M2L (m2l.cu)
 // targets (x charge components) below which a tile's parts run in blocks of their own
@@ -208,6 +215,7 @@ constexpr int64_t kTileSortMin = 512;
 void build_tile_ops(PlanTables& tb, int P, cudaStream_t st);
 bool m2l_tile_supported(const Plan& pl);
 void m2l_tile_setup(Plan& pl);
+void m2l_tile_shard(Plan& pl);
 bool launch_m2l_tile(Plan& pl, const EvalArgs& a, cudaStream_t st);
 // p2p.cu: near-field work items of the plan's tree (leaves with a large near
 // field split into parts), built at plan creation

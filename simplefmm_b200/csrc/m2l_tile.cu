@@ -218,11 +218,24 @@ bool m2l_tile_supported(const Plan& pl)
            !(pl.precision == FMM_PRECISION_MIXED && pl.p >= kTf32MinOrder);
 }
 
-// Tiles of the plan's tree (or of its shard's parents).  pl.sh_list / pl.sh_S
-// hold the split parents level by level.
+// Chunks of at most pl.mt_tpb parents [b, e) per level.
+static void tile_chunks(Plan& pl, Plan::TileList& tl, const std::vector<int32_t>& b, const std::vector<int32_t>& e)
+{
+    std::vector<int4> ck;
+    for (int q = 1; q < pl.tree->depth; ++q)
+        for (int32_t s = b[q]; s < e[q]; s += pl.mt_tpb) ck.push_back(make_int4(s, imin(pl.mt_tpb, e[q] - s), q + 1, 0));
+    tl.chunks = static_cast<int64_t>(ck.size());
+    if (ck.empty()) return;
+    cudaStream_t st = pl.tree->ctx->stream;
+    tl.chunk.alloc(ck.size(), st);
+    SFMM_CUDA(cudaMemcpyAsync(tl.chunk.ptr, ck.data(), ck.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
+}
+
+// Tiles of the plan's tree.  pl.sh_list / pl.sh_S hold the split parents level
+// by level.
 void m2l_tile_setup(Plan& pl)
 {
-    pl.mt_chunks = 0;
+    pl.mt_all.chunks = 0;
     pl.mt_groups = 0;
     pl.mt_on = false;
     if (!m2l_tile_supported(pl)) return;
@@ -254,8 +267,7 @@ void m2l_tile_setup(Plan& pl)
     pl.mt_tpb = 8 * pl.mt_warps / pl.qdim;
     std::vector<int32_t> b(pl.sh_S), e(pl.sh_S);             // per level: parents [b, e)
     for (int q = 1; q < t.depth; ++q) e[q] = pl.sh_S[q + 1];
-    pl.mt_parent.alloc(n, st);
-    const bool shard = pl.shard_count > 1;
+    pl.mt_all.parent.alloc(n, st);
     if (some) {
         // the forest's split parents, those of sparse members apart
         std::vector<int32_t> list(n), tiled, group;
@@ -276,19 +288,10 @@ void m2l_tile_setup(Plan& pl)
         if (!group.empty())
             SFMM_CUDA(cudaMemcpyAsync(pl.mt_group.ptr, group.data(), group.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st));
         if (!tiled.empty())
-            SFMM_CUDA(cudaMemcpyAsync(pl.mt_parent.ptr, tiled.data(), tiled.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st));
+            SFMM_CUDA(cudaMemcpyAsync(pl.mt_all.parent.ptr, tiled.data(), tiled.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st));
         SFMM_CUDA(cudaStreamSynchronize(st));
-    } else if (shard) {
-        std::vector<int32_t> list(n);
-        SFMM_CUDA(cudaMemcpyAsync(list.data(), pl.sh_list.ptr, n * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-        SFMM_CUDA(cudaStreamSynchronize(st));
-        for (int q = 1; q < t.depth; ++q) {
-            const auto lo = list.begin() + pl.sh_S[q], hi = list.begin() + pl.sh_S[q + 1];
-            b[q] = static_cast<int32_t>(std::lower_bound(lo, hi, pl.own_parent_b[q]) - list.begin());
-            e[q] = static_cast<int32_t>(std::lower_bound(lo, hi, pl.own_parent_e[q]) - list.begin());
-        }
     }
-    if (!some && !shard && n >= kTileSortMin) {
+    if (!some && n >= kTileSortMin) {
         DevBuf<uint32_t> k0, k1;
         DevBuf<int64_t> lvl;
         k0.alloc(n, st);
@@ -299,27 +302,44 @@ void m2l_tile_setup(Plan& pl)
                                                                          t.nchild.ptr, k0.ptr);
         SFMM_CHECK_LAUNCH();
         size_t tmp_bytes = 0;
-        SFMM_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, k0.ptr, k1.ptr, pl.sh_list.ptr, pl.mt_parent.ptr,
+        SFMM_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, k0.ptr, k1.ptr, pl.sh_list.ptr, pl.mt_all.parent.ptr,
                                                   static_cast<int>(n), 0, 32, st));
         DevBuf<uint8_t> tmp;
         tmp.alloc(std::max<size_t>(tmp_bytes, 1), st);
-        SFMM_CUDA(cub::DeviceRadixSort::SortPairs(tmp.ptr, tmp_bytes, k0.ptr, k1.ptr, pl.sh_list.ptr, pl.mt_parent.ptr,
+        SFMM_CUDA(cub::DeviceRadixSort::SortPairs(tmp.ptr, tmp_bytes, k0.ptr, k1.ptr, pl.sh_list.ptr, pl.mt_all.parent.ptr,
                                                   static_cast<int>(n), 0, 32, st));
     } else if (!some) {
-        SFMM_CUDA(cudaMemcpyAsync(pl.mt_parent.ptr, pl.sh_list.ptr, n * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
+        SFMM_CUDA(cudaMemcpyAsync(pl.mt_all.parent.ptr, pl.sh_list.ptr, n * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
     }
-    std::vector<int4> ck;
-    for (int q = 1; q < t.depth; ++q)
-        for (int32_t s = b[q]; s < e[q]; s += pl.mt_tpb) ck.push_back(make_int4(s, imin(pl.mt_tpb, e[q] - s), q + 1, 0));
-    pl.mt_chunks = static_cast<int64_t>(ck.size());
-    if (ck.empty()) return;
-    pl.mt_chunk.alloc(ck.size(), st);
-    SFMM_CUDA(cudaMemcpyAsync(pl.mt_chunk.ptr, ck.data(), ck.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
-    const int64_t items = pl.mt_chunks * 8 * (pl.mt_split ? tile::kParts : 1);
+    tile_chunks(pl, pl.mt_all, b, e);
+    if (pl.mt_all.chunks == 0) return;
+    const int64_t items = pl.mt_all.chunks * 8 * (pl.mt_split ? tile::kParts : 1);
     const int64_t blocks = std::min<int64_t>(items, int64_t(sms) * tile::max_per_sm(pl.mt_warps));
     pl.mt_table.alloc(size_t(blocks) * 2 * tile::kSlots * 8 * pl.mt_warps, st);
     pl.mt_part.release();
     if (pl.mt_split) pl.mt_part.alloc(size_t(tile::kParts) * rows * (2 * pl.T + pl.T1), st);
+}
+
+// Tiles of the shard's parents, beside the whole tree's (a captured graph
+// launches on those); slot tables, part sums and widths are the tree's.
+void m2l_tile_shard(Plan& pl)
+{
+    Tree& t = *pl.tree;
+    pl.mt_shard.chunks = 0;
+    const int64_t n = pl.mt_on ? pl.sh_S[t.depth] : 0;
+    if (n == 0) return;
+    cudaStream_t st = t.ctx->stream;
+    std::vector<int32_t> list(n), b(t.depth), e(t.depth);
+    SFMM_CUDA(cudaMemcpyAsync(list.data(), pl.sh_list.ptr, n * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+    SFMM_CUDA(cudaStreamSynchronize(st));
+    for (int q = 1; q < t.depth; ++q) {
+        const auto lo = list.begin() + pl.sh_S[q], hi = list.begin() + pl.sh_S[q + 1];
+        b[q] = static_cast<int32_t>(std::lower_bound(lo, hi, pl.own_parent_b[q]) - list.begin());
+        e[q] = static_cast<int32_t>(std::lower_bound(lo, hi, pl.own_parent_e[q]) - list.begin());
+    }
+    pl.mt_shard.parent.alloc(n, st);
+    SFMM_CUDA(cudaMemcpyAsync(pl.mt_shard.parent.ptr, pl.sh_list.ptr, n * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
+    tile_chunks(pl, pl.mt_shard, b, e);
 }
 
 bool launch_m2l_tile(Plan& pl, const EvalArgs& a, cudaStream_t st)
@@ -332,12 +352,13 @@ bool launch_m2l_tile(Plan& pl, const EvalArgs& a, cudaStream_t st)
         b.m2l_list = pl.mt_group.ptr;
         launch_m2l(b, 0, pl.mt_groups, sms, st);
     }
-    if (pl.mt_chunks == 0) return true;                      // no (other) targets
+    const Plan::TileList& tl = pl.shard_count > 1 ? pl.mt_shard : pl.mt_all;
+    if (tl.chunks == 0) return true;                         // no (other) targets
     tile::TileArgs g{};
     g.ops = pl.tab->tile_ops.ptr;
-    g.parent = pl.mt_parent.ptr;
-    g.chunk = pl.mt_chunk.ptr;
-    g.items = pl.mt_chunks * 8 * (pl.mt_split ? tile::kParts : 1);
+    g.parent = tl.parent.ptr;
+    g.chunk = tl.chunk.ptr;
+    g.items = tl.chunks * 8 * (pl.mt_split ? tile::kParts : 1);
     g.tpb = pl.mt_tpb;
     g.split = pl.mt_split;
     g.node0 = t.lvl_off[2];
@@ -352,7 +373,7 @@ bool launch_m2l_tile(Plan& pl, const EvalArgs& a, cudaStream_t st)
                       : a.p <= 9 ? tile::launch_mid(a, g, pl.mt_warps, sms, st)
                                  : tile::launch_hi(a, g, pl.mt_warps, sms, st);
     if (done && pl.mt_split) {
-        k_tile_sum<<<blocks_for(pl.mt_chunks * 8 * pl.mt_tpb * 32, 256, int64_t(sms) * 16), 256, 0, st>>>(a, g, pl.mt_chunks);
+        k_tile_sum<<<blocks_for(tl.chunks * 8 * pl.mt_tpb * 32, 256, int64_t(sms) * 16), 256, 0, st>>>(a, g, tl.chunks);
         SFMM_CHECK_LAUNCH();
     }
     return done;
