@@ -1,6 +1,7 @@
 // The tiled FP64 M2L kernel (see m2l_tile.cu for the method).
 #pragma once
 
+#include "copy_parity.h"
 #include "m2l_tile.cuh"
 
 namespace sfmm {
@@ -106,6 +107,7 @@ __host__ __device__ constexpr int pad4of8(int n) { return n + (12 - n % 8) % 8; 
 
 constexpr int kRing = 4;                  // D: operators and moments in flight
 constexpr int kOps = 5;                   // operator buffers: R, T, T, I, I; or the D ring
+constexpr int kDrainPolls = 1 << 16;      // of a barrier whose last copy is still in flight when the kernel gives up
 template<int P, int NW>
 struct Smem {
     using F = Frags<P>;
@@ -127,7 +129,8 @@ struct Smem {
     static constexpr int tgt = act + up(2 * kSlots * NW, 16) * 16; // [8 NW] target node of each tile position
     static constexpr int bars = tgt + 4 * 8 * NW;           // mbarriers: kRing per warp (moments); kOps operators full, empty
     static constexpr int misc = bars + 8 * (kRing * NW + 2 * kOps);   // item, slot count, abort
-    static constexpr int total = misc + 16;
+    static constexpr int issued = misc + 16;                // last_copy_parity bits: a byte per warp (moments) and operator buffer
+    static constexpr int total = issued + up(NW + kOps, 8) * 8;
 };
 
 template<int P, int NW>
@@ -148,6 +151,7 @@ __global__ void __launch_bounds__(32 * NW, 1) k_m2l_tile(EvalArgs a, TileArgs g)
     int* ns_s = reinterpret_cast<int*>(sm + S::misc + 8);
     int* abort_s = reinterpret_cast<int*>(sm + S::misc + 12);
     volatile int* abort = abort_s;
+    unsigned char *issM = sm + S::issued + (threadIdx.x >> 5), *issO = sm + S::issued + NW;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, lr = lane >> 2, lc = lane & 3;
     const int qd = a.qdim, tpb = g.tpb;
@@ -156,6 +160,7 @@ __global__ void __launch_bounds__(32 * NW, 1) k_m2l_tile(EvalArgs a, TileArgs g)
     // moments; operators (R, T, I or the D ring) landed; every warp done with them
     uint64_t *barM = bars + warp * kRing, *barO = bars + NW * kRing, *barE = barO + kOps;
     unsigned char *bufM = sm + warp * S::buf_m, *bufZ = sm + S::z + warp * S::buf_z;
+    if (tid < NW + kOps) sm[S::issued + tid] = 0;
     if (tid == 0) {
         for (int i = 0; i < kRing * NW + kOps; ++i) bar_init(bars + i, 1);
         for (int i = 0; i < kOps; ++i) bar_init(barE + i, NW);
@@ -245,13 +250,18 @@ __global__ void __launch_bounds__(32 * NW, 1) k_m2l_tile(EvalArgs a, TileArgs g)
         const int bq = (warp * 8 + (lane & 7)) % qd;
         auto source = [&](int k) { return k < na && lane < 8 ? mine[k * 8 + lane] : -1; };
         // the moments (coefficients [first, first + count)) of those sources into b
-        auto load_moments = [&](int src, unsigned char* b, int first, int count, int stride, uint64_t* bar) {
-            if (lane == 0) bar_expect(bar, 8 * count * 16);
+        auto load_moments = [&](int src, unsigned char* b, int first, int count, int stride, int mb) {
+            uint64_t* bar = barM + mb;
+            if (lane == 0) {
+                *issM ^= 1u << mb;
+                bar_expect(bar, 8 * count * 16);
+            }
             __syncwarp();
             if (lane < 8)
                 bulk(b + lane * stride * 16, src >= 0 ? a.M + (int64_t(src) * qd + bq) * T + first : g.zero, count * 16, bar);
         };
         auto load_ops = [&](int i, int first, int count, int where, int bar) {
+            issO[bar] ^= 1;
             bar_expect(barO + bar, count * 256);
             bulk(sm + where, g.ops + (cls[i] * F::per_class + first) * 32, count * 256, barO + bar);
         };
@@ -339,7 +349,7 @@ __global__ void __launch_bounds__(32 * NW, 1) k_m2l_tile(EvalArgs a, TileArgs g)
                 fresh = false;
             };
             int k = 0;                                      // the warp's next slot
-            if (na > 0) load_moments(source(0), bufM, 0, F::TW, CS, barM);
+            if (na > 0) load_moments(source(0), bufM, 0, F::TW, CS, 0);
             int src = source(1);                            // sources of the slot after it
             if (ns > 0 && tid == 0) {
                 load_ops(0, 0, F::NR, S::ops, 0);
@@ -427,7 +437,7 @@ __global__ void __launch_bounds__(32 * NW, 1) k_m2l_tile(EvalArgs a, TileArgs g)
                 }
                 done(0);
                 if (on && k < na) {                         // the moments are used up: the next slot's
-                    load_moments(src, bufM, 0, F::TW, CS, barM);
+                    load_moments(src, bufM, 0, F::TW, CS, 0);
                     src = source(k + 1);
                     load_e();
                 }
@@ -546,7 +556,7 @@ __global__ void __launch_bounds__(32 * NW, 1) k_m2l_tile(EvalArgs a, TileArgs g)
             proxy_fence();                                   // the stages wrote this space through the generic proxy
             // moments kRing slots ahead, their sources one more
             for (int u = 0; u < kRing; ++u)
-                if (u < na) load_moments(source(u), ring + u * S::ring_m, F::TW, P + 1, CD, barM + u);
+                if (u < na) load_moments(source(u), ring + u * S::ring_m, F::TW, P + 1, CD, u);
             int src = source(kRing);
             if (tid == 0)
                 for (int u = 0; u < kRing && u < ns; ++u) load_ops(u, first, F::ND, S::ops_d + u * 256 * F::ND, u);
@@ -609,7 +619,7 @@ __global__ void __launch_bounds__(32 * NW, 1) k_m2l_tile(EvalArgs a, TileArgs g)
                     }
                     // the moments are used up: those kRing slots later take their place
                     __syncwarp();
-                    if (k + kRing - 1 < na) load_moments(src, ring + mb * S::ring_m, F::TW, P + 1, CD, barM + mb);
+                    if (k + kRing - 1 < na) load_moments(src, ring + mb * S::ring_m, F::TW, P + 1, CD, mb);
                     src = source(k + kRing);
                 }
                 done(b);
@@ -627,15 +637,12 @@ __global__ void __launch_bounds__(32 * NW, 1) k_m2l_tile(EvalArgs a, TileArgs g)
         __syncthreads();
         if (*abort) {
             // copies in flight land before shared memory is released
-            if (lane == 0)
-                for (int b = 0; b < kRing; ++b)
-                    for (long it = 0; it < (1L << 20) && !(bar_try(barM + b, 0) && bar_try(barM + b, 1)); ++it) {
-                    }
+            if (lane == 0) drain_copies(*issM, kRing, kDrainPolls, [&](int b, uint32_t parity) { return bar_try(barM + b, parity); });
             if (tid == 0) {
                 atomicExch(a.wait_err, 1);
-                for (int b = 0; b < kOps; ++b)
-                    for (long it = 0; it < (1L << 20) && !(bar_try(barO + b, 0) && bar_try(barO + b, 1)); ++it) {
-                    }
+                uint32_t issued = 0;
+                for (int b = 0; b < kOps; ++b) issued |= uint32_t(issO[b]) << b;
+                drain_copies(issued, kOps, kDrainPolls, [&](int b, uint32_t parity) { return bar_try(barO + b, parity); });
             }
             break;
         }
