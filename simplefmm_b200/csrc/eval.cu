@@ -552,10 +552,12 @@ void plan_init(Plan& pl)
     pl.m2l_ctr.alloc(1, st);
     pl.wait_err.alloc(1, st);
     SFMM_CUDA(cudaMemsetAsync(pl.wait_err.ptr, 0, sizeof(int32_t), st));
-    // test switch: the row-owner M2L kernel instead of the tensor-core ones
+    // test switch: the row-owner M2L kernel instead of the tensor-core ones, the
+    // rotation M2L of mixed plans, or tiles whose parts never run apart
     const char* mk = std::getenv("SFMM_M2L_KERNEL");
     pl.m2l_force_rows = mk && std::strcmp(mk, "rows") == 0;
     pl.m2l_rotation_only = mk && std::strcmp(mk, "rotation") == 0;
+    pl.m2l_whole_tiles = mk && std::strcmp(mk, "whole") == 0;
     const int kmax = pl.qdim + 3;
     pl.qs.alloc(size_t(t.n) * pl.qdim, st);
     if (pl.precision == FMM_PRECISION_FP64) {

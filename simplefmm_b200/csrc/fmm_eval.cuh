@@ -163,6 +163,7 @@ struct Plan {
     DevBuf<int32_t> mt_group;                 // a forest's parents of sparse members: the group kernel takes them
     int64_t mt_groups = 0;
     bool m2l_force_rows = false;              // SFMM_M2L_KERNEL=rows at plan creation
+    bool m2l_whole_tiles = false;             // SFMM_M2L_KERNEL=whole: a tile's parts never in blocks of their own
     int m2l_method = FMM_M2L_METHOD_ROTATION;        // fmm_plan_set_m2l
     // sharded evaluation (fmm_plan_set_shard): this plan's share of one solve
     int shard_index = 0, shard_count = 1;

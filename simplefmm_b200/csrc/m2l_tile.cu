@@ -262,7 +262,7 @@ void m2l_tile_setup(Plan& pl)
     // and 1.92 ms; p = 6, 60k 0.57, 0.46 and 0.46 ms)
     const int64_t rows = (t.lvl_off[t.depth + 1] - t.lvl_off[2]) * pl.qdim;
     const int full = tile::full_warps(pl.p);
-    pl.mt_split = rows < kTileSplitRows;
+    pl.mt_split = rows < kTileSplitRows && !pl.m2l_whole_tiles;
     pl.mt_warps = pl.mt_split && rows * tile::kParts < int64_t(sms) * 2 * 8 * full ? tile::kSmallWarps : full;
     pl.mt_tpb = 8 * pl.mt_warps / pl.qdim;
     std::vector<int32_t> b(pl.sh_S), e(pl.sh_S);             // per level: parents [b, e)

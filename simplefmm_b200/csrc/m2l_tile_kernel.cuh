@@ -90,6 +90,10 @@ __device__ __forceinline__ double2 lds2(uint32_t addr)
     return v;
 }
 
+// o + u s with both roundings, so that a part's share is the same number whether
+// it is added here or stored and added by k_tile_sum.
+__device__ __forceinline__ double add_scaled(double o, double u, double s) { return __dadd_rn(o, __dmul_rn(u, s)); }
+
 // The loads that v depends on stay before this point.
 __device__ __forceinline__ void before(double (&v)[4])
 {
@@ -338,7 +342,7 @@ __global__ void __launch_bounds__(32 * NW, 1) k_m2l_tile(EvalArgs a, TileArgs g)
                                     const int m = 8 * rt + lr;
                                     const double(&u)[4] = sum[u0 + rt];
                                     const cplx o = old[u0 + rt - first];
-                                    if (m <= j) out[j * (j + 1) / 2 + m] = cplx{o.re + u[h] * sc, o.im + u[2 + h] * sc};
+                                    if (m <= j) out[j * (j + 1) / 2 + m] = cplx{add_scaled(o.re, u[h], sc), add_scaled(o.im, u[2 + h], sc)};
                                 }
                             }
                         });
@@ -545,7 +549,8 @@ __global__ void __launch_bounds__(32 * NW, 1) k_m2l_tile(EvalArgs a, TileArgs g)
 #pragma unroll
                     for (int t = 0; t < F::DT; ++t) {
                         const double sc = lvl[order[t] + 1];
-                        if (8 * t + lr < T) out[8 * t + lr] = cplx{old[t].re + sum[t][h] * sc, old[t].im + sum[t][2 + h] * sc};
+                        if (8 * t + lr < T)
+                            out[8 * t + lr] = cplx{add_scaled(old[t].re, sum[t][h], sc), add_scaled(old[t].im, sum[t][2 + h], sc)};
                     }
                 }
 #pragma unroll
