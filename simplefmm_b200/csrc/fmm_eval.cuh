@@ -3,6 +3,7 @@
 
 #include "fmm_internal.cuh"
 #include "i8_ops.h"
+#include "tile_parts.h"
 
 #include <memory>
 
@@ -206,10 +207,7 @@ void shift_l2l(Plan& pl, const EvalArgs& a, int lc, cudaStream_t st);
 // m2l_tile.cu: the FP64 M2L of orders kTileMinOrder..kTileMaxOrder; operators
 // per (device, p), set-up per plan (after shift_setup), the tiles of a shard's
 // parents (plan_set_shard), launch (false: the plan takes another kernel)
-constexpr int kTileMinOrder = 2, kTileMaxOrder = 12;
 constexpr int kTf32MinOrder = 11;         // lowest order at which mixed plans use the TF32 M2L (m2l.cu)
-// targets (x charge components) below which a tile's parts run in blocks of their own
-constexpr int64_t kTileSplitRows = 24 * 1024;
 // parents from which on they are sorted by the pattern of their neighbours (25 us of set-up; 100,000 uniform points,
 // p = 8, 585 parents: M2L 0.81 -> 0.72 ms)
 constexpr int64_t kTileSortMin = 512;

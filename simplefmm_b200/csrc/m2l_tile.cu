@@ -218,6 +218,21 @@ bool m2l_tile_supported(const Plan& pl)
            !(pl.precision == FMM_PRECISION_MIXED && pl.p >= kTf32MinOrder);
 }
 
+// Room for the part sums of `rows` rows; false (the parts then run in turn, to
+// the same sums) where the device has too little.
+static bool take_parts(Plan& pl, int64_t rows)
+{
+    const size_t bytes = tile_part_bytes(rows, pl.p);
+    if (rows >= kTileSplitRows || pl.m2l_whole_tiles) return false;
+    try {
+        pl.mt_part.alloc(coarse_bytes(bytes) / sizeof(double2), pl.tree->ctx->stream);
+    } catch (const Error& e) {
+        if (e.status != FMM_ERR_OUT_OF_MEMORY) throw;
+        return false;
+    }
+    return true;
+}
+
 // Chunks of at most pl.mt_tpb parents [b, e) per level.
 static void tile_chunks(Plan& pl, Plan::TileList& tl, const std::vector<int32_t>& b, const std::vector<int32_t>& e)
 {
@@ -262,7 +277,7 @@ void m2l_tile_setup(Plan& pl)
     // and 1.92 ms; p = 6, 60k 0.57, 0.46 and 0.46 ms)
     const int64_t rows = (t.lvl_off[t.depth + 1] - t.lvl_off[2]) * pl.qdim;
     const int full = tile::full_warps(pl.p);
-    pl.mt_split = rows < kTileSplitRows && !pl.m2l_whole_tiles;
+    pl.mt_split = take_parts(pl, rows);
     pl.mt_warps = pl.mt_split && rows * tile::kParts < int64_t(sms) * 2 * 8 * full ? tile::kSmallWarps : full;
     pl.mt_tpb = 8 * pl.mt_warps / pl.qdim;
     std::vector<int32_t> b(pl.sh_S), e(pl.sh_S);             // per level: parents [b, e)
@@ -315,9 +330,7 @@ void m2l_tile_setup(Plan& pl)
     if (pl.mt_all.chunks == 0) return;
     const int64_t items = pl.mt_all.chunks * 8 * (pl.mt_split ? tile::kParts : 1);
     const int64_t blocks = std::min<int64_t>(items, int64_t(sms) * tile::max_per_sm(pl.mt_warps));
-    pl.mt_table.alloc(size_t(blocks) * 2 * tile::kSlots * 8 * pl.mt_warps, st);
-    pl.mt_part.release();
-    if (pl.mt_split) pl.mt_part.alloc(size_t(tile::kParts) * rows * (2 * pl.T + pl.T1), st);
+    pl.mt_table.alloc(coarse_bytes(size_t(blocks) * 2 * tile::kSlots * 8 * pl.mt_warps * sizeof(int32_t)) / sizeof(int32_t), st);
 }
 
 // Tiles of the shard's parents, beside the whole tree's (a captured graph

@@ -12,7 +12,7 @@ namespace tile {
 
 constexpr int kSlots = 216;               // offsets of an octant: a 6 x 6 x 6 box around the target
 constexpr int kClasses = 70;              // rotation classes (fmm.hpp:169)
-constexpr int kParts = 6;                 // parts of the slots: the planes of one y offset, 36 slots each
+constexpr int kParts = kTileParts;        // parts of the slots: the planes of one y offset, 36 slots each
 constexpr int kPartSlots = kSlots / kParts;
 constexpr int kSmallWarps = 2;            // warps of a block when there are few tiles
 
