@@ -55,6 +55,7 @@
 #include <cub/device/device_radix_sort.cuh>
 
 #include <algorithm>
+#include <cstdint>
 #include <vector>
 
 #include "m2l_tile.cuh"
@@ -218,14 +219,18 @@ bool m2l_tile_supported(const Plan& pl)
            !(pl.precision == FMM_PRECISION_MIXED && pl.p >= kTf32MinOrder);
 }
 
+static thread_local size_t tl_part_limit = SIZE_MAX;
+
+void set_thread_tile_part_limit(size_t bytes) noexcept { tl_part_limit = bytes; }
+
 // Room for the part sums of `rows` rows; false (the parts then run in turn, to
-// the same sums) where the device has too little.
+// the same sums) where the thread's limit or the device has too little.
 static bool take_parts(Plan& pl, int64_t rows)
 {
     const size_t bytes = tile_part_bytes(rows, pl.p);
-    if (rows >= kTileSplitRows || pl.m2l_whole_tiles) return false;
+    if (rows >= kTileSplitRows || pl.m2l_whole_tiles || bytes > tl_part_limit) return false;
     try {
-        pl.mt_part.alloc(coarse_bytes(bytes) / sizeof(double2), pl.tree->ctx->stream);
+        pl.mt_part.alloc(std::min(coarse_bytes(bytes), tl_part_limit) / sizeof(double2), pl.tree->ctx->stream);
     } catch (const Error& e) {
         if (e.status != FMM_ERR_OUT_OF_MEMORY) throw;
         return false;

@@ -17,7 +17,8 @@
 // and a server's workers bypass the library's block cache, so freed blocks go
 // back to the pool: fmm_server_memory reports the measured peak of the
 // running requests' device memory beside the budget, and the largest ratio
-// of a request's measured peak to its estimate.
+// of a request's measured peak to its estimate.  The part sums of small FP64
+// solves (tile_parts.h) come on top, where the budget has room for them.
 //
 // Leaf size: a request may name max_particles_per_node, or pass 0 to let the
 // server's autotuner choose: per (p, precision, log2 N) bucket it tries each
@@ -55,6 +56,7 @@
 #include "alloc_meter.h"
 #include "i8_ops.h"
 #include "simplefmm_b200.h"
+#include "tile_parts.h"
 
 namespace sfmm {
 int record_failure(int status, const char* msg);
@@ -72,7 +74,8 @@ struct Request {
     int qdim = 1, p = 0, precision = 0, leaf = 0;
     double* pot = nullptr;
     double* field = nullptr;
-    size_t bytes = 0;                 // estimated device memory (admission)
+    size_t bytes = 0;                 // estimated device memory (admission), and what it was given for part sums
+    size_t parts = 0;                 // bytes of part sums its M2L can use (tile_parts.h)
     int64_t measured = 0;             // measured peak of its device allocations
     bool tuned = false;               // leaf size chosen by the autotuner
     Clock::time_point t_submit, t_done;
@@ -99,8 +102,6 @@ size_t estimate_bytes(int64_t n, int p, int qdim, int leaf, int precision)
     // are first allocated for n / 8 nodes (15 B per point)
     const double per_point = 48 + 48 + 48 + 8.0 * (qdim + 3) * 3 + 16;
     double per_node = 16.0 * qdim * (2 * T + T1) + 190 * 8 + 64;         // M, LA, LB, ilist, node arrays
-    // the tiled FP64 M2L of small trees: the parts' sums
-    if (precision == FMM_PRECISION_FP64 && nodes * qdim < 24 * 1024) per_node += 6 * 16.0 * qdim * (2 * T + T1);
     // mixed plans' tensor-core M2L (m2l_i8.cu): slot table, block lists and
     // four digits of the padded real moments per node
     if (precision == FMM_PRECISION_MIXED && p <= sfmm::kI8MaxOrder)
@@ -158,6 +159,7 @@ struct fmm_server {
     std::unordered_map<int64_t, std::shared_ptr<Request>> all;
     size_t in_use = 0, peak_in_use = 0;
     int running = 0, peak_running = 0;
+    int busy = 0;                         // workers with requests
     sfmm::AllocMeter meter;               // measured device bytes of the running requests
     double worst_ratio = 0;               // largest measured / estimated over completed requests
     int64_t next_id = 1;
@@ -167,10 +169,27 @@ struct fmm_server {
     Autotuner tuner;
 
     void worker(int slot);
+    size_t grant_parts(const std::vector<std::shared_ptr<Request>>& rs) const;
     void run(fmm_context* c, Request& r);
     void run_batch(fmm_context* c, std::vector<std::shared_ptr<Request>>& rs);
     void finish(Request& r);
 };
+
+// Bytes of part sums for requests just admitted together (mu held): what they
+// can use, if that fits beside the running requests and the queued ones that
+// the idle workers could take; else none.  A request is never refused or kept
+// waiting for part sums: without them its M2L runs a tile's parts in turn, to
+// the same results.
+size_t fmm_server::grant_parts(const std::vector<std::shared_ptr<Request>>& rs) const
+{
+    size_t want = 0;
+    for (const auto& r : rs) want += r->parts;
+    want = std::min(want, sfmm::coarse_bytes(sfmm::tile_part_bytes(sfmm::kTileSplitRows, rs[0]->p)));
+    size_t used = in_use;
+    const size_t idle = ctx.size() - size_t(busy) - 1;     // beside the worker that asks
+    for (size_t i = 0; i < std::min(idle, queue.size()); ++i) used += queue[i]->bytes;
+    return used + want <= budget ? want : 0;
+}
 
 void fmm_server::run_batch(fmm_context* c, std::vector<std::shared_ptr<Request>>& rs)
 {
@@ -262,6 +281,11 @@ void fmm_server::worker(int slot)
                 ++batches;
                 batched += int64_t(rs.size());
             }
+            const size_t parts = grant_parts(rs);
+            sfmm::set_thread_tile_part_limit(parts);
+            rs[0]->bytes += parts;
+            in_use += parts;
+            ++busy;
             peak_in_use = std::max(peak_in_use, in_use);
             running += int(rs.size());
             peak_running = std::max(peak_running, running);
@@ -271,6 +295,7 @@ void fmm_server::worker(int slot)
         {
             std::lock_guard<std::mutex> lk(mu);
             for (auto& r : rs) finish(*r);
+            --busy;
         }
         cv_done.notify_all();
         cv_work.notify_all();
@@ -339,6 +364,7 @@ int fmm_server_submit(fmm_server* s, const double* xyz, int64_t n, const double*
     if (r->bytes > s->budget)
         return sfmm::record_failure(FMM_ERR_OVER_BUDGET, "request's estimated device memory exceeds the server budget");
     if (r->tuned) r->leaf = s->tuner.choose(*r);
+    if (precision == FMM_PRECISION_FP64) r->parts = sfmm::tile_part_estimate(n, r->leaf, qdim, p);
     {
         std::lock_guard<std::mutex> lk(s->mu);
         if (s->stopping) return sfmm::record_failure(FMM_ERR_INVALID_ARGUMENT, "server is stopping");

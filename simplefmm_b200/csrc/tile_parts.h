@@ -1,7 +1,9 @@
-// Device memory of the tiled FP64 M2L's part sums (m2l_tile.cu; pure C++,
-// shared with a CPU test).
+// Device memory of the tiled FP64 M2L's part sums (m2l_tile.cu): what a plan
+// takes and what the serving loop sets aside for it (pure C++, shared with a
+// CPU test).
 #pragma once
 
+#include <algorithm>
 #include <cstddef>
 #include <cstdint>
 
@@ -36,5 +38,23 @@ inline size_t tile_part_bytes(int64_t rows, int p)
     const size_t T = (p + 1) * (p + 2) / 2, T1 = (p + 2) * (p + 3) / 2;
     return size_t(kTileParts) * 16 * (2 * T + T1) * size_t(rows);
 }
+
+// What to set aside for the part sums of n points with leaves of at most
+// `leaf`.  A node that splits has more than `leaf` points and eight children at
+// most, so a tree of even depth has up to 64/7 n / leaf nodes (measured: 40,000
+// uniform points, leaf 64, 7.1 n / leaf; 300,007 Plummer points 4.0); a plan
+// whose rows need more than it was given runs its parts in turn.  Leaves are at
+// least n / leaf, so large trees take none.
+inline size_t tile_part_estimate(int64_t n, int leaf, int qdim, int p)
+{
+    if (p < kTileMinOrder || p > kTileMaxOrder) return 0;
+    const int64_t leaves = n / std::max(leaf, 1);
+    if (leaves * qdim >= kTileSplitRows) return 0;
+    return coarse_bytes(tile_part_bytes(std::min<int64_t>((64 * leaves / 7 + 128) * qdim, kTileSplitRows), p));
+}
+
+// Most bytes of part sums that plans made by the calling thread may take
+// (m2l_tile.cu; the serving loop sets it for its requests).  No limit at first.
+void set_thread_tile_part_limit(size_t bytes) noexcept;
 
 }  // namespace sfmm
