@@ -493,10 +493,14 @@ static void evaluate_graph(sfmm::Plan& pl, const double* Q, double* pot, double*
     }
     SFMM_CUDA(cudaStreamEndCapture(c.stream, &g));
     // launch shape: the kernel sequence depends on the depth, the order, the
-    // precision, the charge components and the outputs
+    // precision, the charge components, the outputs, on which M2L the members
+    // take (tiles, the group kernel, both; a tile's parts apart add a sum) and on
+    // whether some leaf's near field runs in parts
     const uint64_t shape = uint64_t(pl.tree->depth) | uint64_t(pl.p) << 8 | uint64_t(pl.precision) << 16 |
                            uint64_t(pl.qdim) << 20 | uint64_t(pot != nullptr) << 24 | uint64_t(field != nullptr) << 25 |
-                           uint64_t(pl.i8 != nullptr) << 26;
+                           uint64_t(pl.i8 != nullptr) << 26 | uint64_t(pl.mt_on) << 27 | uint64_t(pl.mt_split) << 28 |
+                           uint64_t(pl.mt_groups > 0) << 29 | uint64_t(pl.mt_all.chunks > 0) << 30 |
+                           uint64_t(pl.p2p_rows > 0) << 31;
     cudaGraphExec_t exec = nullptr;
     for (auto& e : c.batch_graphs)
         if (e.first == shape) {
