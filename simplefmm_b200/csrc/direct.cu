@@ -57,6 +57,35 @@ __device__ __forceinline__ void direct_tile(const double4* __restrict__ s4, cons
     }
 }
 
+// A target's field again, from the unit vectors R / r: q / r^3 leaves the range
+// of the type where q / r^2 does not (pairs closer than 1e-102, say, or charges
+// of 1e-150 at 1e60).  Only targets whose potential is finite and whose field is
+// not, or whose potential is below 1e-90, come here: q / r^3 below the type's
+// normal numbers means q / r below 1e-102 for every r whose cube is in range.
+template<int QD>
+__device__ __noinline__ void direct_field_in_range(const double* __restrict__ xyz, const double* __restrict__ Q, int64_t jb, int64_t je,
+                                                   int64_t i, double (&f)[3])
+{
+    const double x = xyz[3 * i], y = xyz[3 * i + 1], z = xyz[3 * i + 2];
+    f[0] = f[1] = f[2] = 0.0;
+    for (int64_t j = jb; j < je; ++j) {
+        if (j == i) continue;
+        const double dx = x - xyz[3 * j], dy = y - xyz[3 * j + 1], dz = z - xyz[3 * j + 2];
+        const double r = sqrt(fma(dx, dx, fma(dy, dy, dz * dz)));
+        const double ex = dx / r, ey = dy / r, ez = dz / r;
+        const double* q = Q + j * QD;
+        if (QD == 1) {
+            f[0] += q[0] / r * ex / r;
+            f[1] += q[0] / r * ey / r;
+            f[2] += q[0] / r * ez / r;
+        } else if (QD == 3) {
+            f[0] += (q[1] * ez - q[2] * ey) / r / r;
+            f[1] += (q[2] * ex - q[0] * ez) / r / r;
+            f[2] += (q[0] * ey - q[1] * ex) / r / r;
+        }
+    }
+}
+
 template<int QD>
 __global__ void __launch_bounds__(kThreads) k_direct(const double* __restrict__ xyz, int64_t n, const double* __restrict__ Q,
                                                      const int64_t* __restrict__ targets, int64_t nt, int64_t chunk,
@@ -104,6 +133,12 @@ __global__ void __launch_bounds__(kThreads) k_direct(const double* __restrict__ 
 #pragma unroll
     for (int u = 0; u < kPerThread; ++u) {
         if (!on[u]) continue;
+        double ps = 0.0;
+#pragma unroll
+        for (int b = 0; b < QD; ++b) ps += fabs(pa[u][b]);
+        const bool in_range = isfinite(fa[u][0]) && isfinite(fa[u][1]) && isfinite(fa[u][2]);
+        if (QD != 2 && isfinite(ps) && (!in_range || (ps > 0.0 && ps < 1e-90)))
+            direct_field_in_range<QD>(xyz, Q, jb, je, i[u], fa[u]);
         double* o = part + (blockIdx.y * nt + t[u]) * 6;
         for (int b = 0; b < 3; ++b) o[b] = b < QD ? pa[u][b < QD ? b : 0] : 0.0;
         for (int c = 0; c < 3; ++c) o[3 + c] = fa[u][c];
