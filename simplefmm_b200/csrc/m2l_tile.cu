@@ -279,11 +279,14 @@ void m2l_tile_setup(Plan& pl)
     if (n == 0) return;
     // few targets: the parts of a tile in blocks of their own, and if that does not give every SM two full blocks to
     // run one after the other, narrow tiles (p = 10 at one, two and four blocks, M2L: Plummer 100k points 1.35, 1.35
-    // and 1.92 ms; p = 6, 60k 0.57, 0.46 and 0.46 ms)
+    // and 1.92 ms; p = 6, 60k 0.57, 0.46 and 0.46 ms).  From order 11 on one narrow block's operators
+    // fill an SM (119 KB of shared memory), two warps, and full blocks are faster: M2L at p = 12, narrow and full, of
+    // Plummer 20k points 1.56 and 1.13 ms, 10k in leaves of 32 1.43 and 0.98; whole evaluations of 41 small trees,
+    // full / narrow in the mean 0.80 at p = 11 and 0.84 at 12 (0.61 to 1.04), but 1.14 at 6, 1.13 at 8, 1.03 at 10
     const int64_t rows = (t.lvl_off[t.depth + 1] - t.lvl_off[2]) * pl.qdim;
     const int full = tile::full_warps(pl.p);
     pl.mt_split = take_parts(pl, rows);
-    pl.mt_warps = pl.mt_split && rows * tile::kParts < int64_t(sms) * 2 * 8 * full ? tile::kSmallWarps : full;
+    pl.mt_warps = pl.mt_split && pl.p <= tile::kNarrowMaxOrder && rows * tile::kParts < int64_t(sms) * 2 * 8 * full ? tile::kSmallWarps : full;
     pl.mt_tpb = 8 * pl.mt_warps / pl.qdim;
     std::vector<int32_t> b(pl.sh_S), e(pl.sh_S);             // per level: parents [b, e)
     for (int q = 1; q < t.depth; ++q) e[q] = pl.sh_S[q + 1];

@@ -14,7 +14,8 @@ constexpr int kSlots = 216;               // offsets of an octant: a 6 x 6 x 6 b
 constexpr int kClasses = 70;              // rotation classes (fmm.hpp:169)
 constexpr int kParts = kTileParts;        // parts of the slots: the planes of one y offset, 36 slots each
 constexpr int kPartSlots = kSlots / kParts;
-constexpr int kSmallWarps = 2;            // warps of a block when there are few tiles
+constexpr int kSmallWarps = 2;            // warps of a block when there are few tiles, orders up to kNarrowMaxOrder
+constexpr int kNarrowMaxOrder = 10;
 
 // |d|^2 of a rotation class (class = 7 t2i + dk + 3, fmm.hpp:171)
 __host__ __device__ inline int class_dist2(int c)

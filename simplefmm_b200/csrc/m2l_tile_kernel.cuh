@@ -674,7 +674,9 @@ bool launch_w(const EvalArgs& a, const TileArgs& g, int sms, cudaStream_t st)
 template<int P>
 bool launch_p(const EvalArgs& a, const TileArgs& g, int warps, int sms, cudaStream_t st)
 {
-    return warps == kSmallWarps ? launch_w<P, kSmallWarps>(a, g, sms, st) : launch_w<P, full_warps(P)>(a, g, sms, st);
+    if constexpr (P <= kNarrowMaxOrder)
+        if (warps == kSmallWarps) return launch_w<P, kSmallWarps>(a, g, sms, st);
+    return launch_w<P, full_warps(P)>(a, g, sms, st);
 }
 
 }  // namespace tile
