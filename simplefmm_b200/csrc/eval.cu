@@ -65,6 +65,10 @@ __global__ void k_gather_q(const double* __restrict__ Q, const int32_t* __restri
 // 10 to 30 points a leaf): p = 10, 300k points 78 -> 60 us, 1M 223 -> 170; p = 12,
 // 16M points 2.82 -> 2.18 ms.  Two points a lane for more independent chains took
 // 128 registers and was slower (1M 201 us).
+//
+// Charge components take a pass over the leaf each, powers and recurrences
+// anew: 300k Plummer points, three components, 245 -> 184 us at p = 12, 120 ->
+// 106 at 8, 79 -> 73 at 6, but 37 -> 44 at p = 3.
 __host__ __device__ constexpr int lanes_per_point(int p) { return p / 2 + 1; }
 
 // Step j of lane i: (n, m); false for the middle order's unused second half.
@@ -690,9 +694,13 @@ void plan_evaluate(Plan& pl, const double* Q, double* pot, double* field, cudaEv
     SFMM_CHECK_LAUNCH();
     SFMM_CUDA(cudaMemsetAsync(pl.out.ptr, 0, size_t(t.n) * K * sizeof(double), st));
     // The near field (P2P) depends only on the points and the gathered charges:
-    // it runs on the context's side stream, issued after the M2L so that the
-    // M2L's blocks are dispatched first and the near field fills the M2L's
-    // tail and the downward pass; the stream joins back before the sums.
+    // it runs on the context's side stream from the fork on, beside the upward
+    // pass, and the stream joins back before the sums.  On large trees nothing
+    // is won by that: the near field fills the GPU, the upward pass takes as long
+    // as it (4M Plummer, p = 10: 9.3 ms for 1.4 ms of kernels), and a block of
+    // the tiled or the int8 M2L leaves no room on its SM for another (the step's
+    // 50.4 ms are the sum of its kernels' times).  On small trees the launches
+    // of both chains overlap.
     SFMM_CUDA(cudaEventRecord(pl.fork, st));
     cudaStream_t side = t.ctx->side ? t.ctx->side : st;
     auto near_field = [&] {

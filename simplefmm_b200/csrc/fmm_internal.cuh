@@ -251,6 +251,13 @@ struct Tree {
 // ms, 400k (42) 3.5 / 2.8; Plummer 20k (90) 0.59 / 1.06, 400k (150) 4.5 / 7.2.
 // Trees of a few hundred targets are latency-bound and faster tiled: shell
 // 3,000 points (26) 0.24 / 0.27, uniform 3,000 (38) 0.25 / 0.30.
+// Other orders and components, shell: 60k points p = 6 0.59 / 0.38, p = 12 1.82 /
+// 1.01; three components 60k p = 8 1.30 / 1.18, 400k p = 6 3.5 / 3.1.  The line is
+// not exact: three components at 400k are even (p = 8 5.3 / 5.8, p = 12 14.2 /
+// 14.5), shells of 1,000 to 2,000 targets at p <= 8 up to a third faster tiled (20k
+// points, p = 7, three components 0.40 / 0.64), and scalar charges at p = 11 and 12
+// on 200 to 400 targets with under 45 sources faster by the group kernel
+// (Plummer 2,000 points, p = 12 0.50 / 0.33).
 inline bool m2l_sparse(int64_t pairs, int64_t targets) { return targets >= 1024 && pairs < 56 * targets; }
 
 struct Plan;

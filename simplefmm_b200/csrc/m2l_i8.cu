@@ -59,7 +59,9 @@
 // a thread of its own and two K steps per set of barrier waits brought a step
 // to 995 cycles (shared rows: 12 instead of 18 steps a slot), 19.3 ms, against
 // 640 cycles of MMA.  TMA gathers of the rows (tile::gather4) took 2450 cycles
-// a step.  1M Plummer points, p = 10: 7.1 -> 3.8 ms.
+// a step.  1M Plummer points, p = 10: 7.1 -> 3.8 ms; there the tensor pipe is
+// active 63% of the time, L2 at 28% of its throughput and an SM receives 24
+// bytes a cycle, so neither is full: the rest is the hand-over of stages.
 //
 // Roles (one block per SM, persistent over the items): warps 0-3 gather the
 // moment rows (cp.async) and issue the operator bulk copies; the relay thread

@@ -97,7 +97,9 @@ struct Frags {
 };
 
 // Warps of a full block: as many as the sums' registers (8 per row tile) and
-// the operand buffers in shared memory leave room for.
+// the operand buffers in shared memory leave room for.  At 255 registers some
+// of it is still spilled: 80 bytes a thread at p = 10, 190 at 11, 270 at 8, 1,070
+// at 12.
 __host__ __device__ constexpr int full_warps(int P) { return P <= 6 ? 16 : P <= 8 ? 12 : P <= 10 ? 8 : 6; }
 
 // resident blocks per SM at most (the blocks' slot tables are sized for them)

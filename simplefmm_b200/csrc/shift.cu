@@ -19,9 +19,10 @@
 //              per block, a warp per octant: each sums its octant's products on
 //              the FP64 tensor cores (mma.sync m8n8k4, both operands read from
 //              L2), then the eight are added in octant order.  A level is a
-//              chain of at most 39 K chunks whatever its size; one warp taking
-//              the eight octants in turn (32 columns a block, the children
-//              staged per octant) took 90 us for a level of a few boxes.
+//              chain of ceil((p+1)(p+2)/4) K chunks whatever its size (33 at
+//              p = 10, 46 at 12, 77 at 16); one warp taking the eight octants in
+//              turn (32 columns a block, the children staged per octant) took
+//              90 us for a level of a few boxes.
 //   k_l2l_mma  stages the parents' locals, and for each 8-row tile of OpL adds
 //              the product into the child of that row's octant (each child
 //              coefficient has one writer: no atomics, deterministic); 64
