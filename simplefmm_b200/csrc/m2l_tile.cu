@@ -164,21 +164,34 @@ __global__ void k_tile_keys(const int32_t* __restrict__ list, int64_t n, const i
     }
 }
 
-// Split tiles: the parts' sums added in part order, a warp per target.
+// Split tiles: the parts' sums scaled to the level and added in part order as
+// the kernel does where one block has them all, a warp per target.
 __global__ void k_tile_sum(EvalArgs a, tile::TileArgs g, int64_t chunks)
 {
     const int lane = threadIdx.x & 31, qd = a.qdim;
     const int64_t stride = (int64_t(gridDim.x) * blockDim.x) >> 5, total = chunks * 8 * g.tpb;
-    // the part sums of len coefficients from `first` on, then (more) the order-P sources'
-    auto sum = [&](const cplx* part, const cplx* more, int64_t first, int64_t len, cplx* out) {
-        for (int64_t e = lane; e < len; e += 32) {
-            cplx v = part[first + e];
+    // the part sums of qd rows of `len` coefficients, then (more) the order-P sources'; lane j holds the scale of order j
+    auto sum = [&](const cplx* part, const cplx* more, int64_t row, int len, double scale, cplx* out) {
+        for (int e0 = 0; e0 < qd * len; e0 += 32) {
+            const int e = e0 + lane;
+            const bool on = e < qd * len;
+            cplx w[2 * tile::kParts];
 #pragma unroll
-            for (int q = 1; q < 2 * tile::kParts; ++q) {
+            for (int q = 0; q < 2 * tile::kParts; ++q) {
                 if (q >= tile::kParts && !more) break;
-                const cplx w = (q < tile::kParts ? part : more)[(q % tile::kParts) * g.rows * (len / qd) + first + e];
-                v.re += w.re;
-                v.im += w.im;
+                if (on) w[q] = (q < tile::kParts ? part : more)[((q % tile::kParts) * g.rows + row) * len + e];
+            }
+            int c = e, j, m;
+            while (c >= len) c -= len;
+            tri_nm(c, j, m);
+            const double sc = __shfl_sync(0xffffffffu, scale, j);
+            if (!on) continue;
+            cplx v{0, 0};
+#pragma unroll
+            for (int q = 0; q < 2 * tile::kParts; ++q) {
+                if (q >= tile::kParts && !more) break;
+                v.re = fma(w[q].re, sc, v.re);
+                v.im = fma(w[q].im, sc, v.im);
             }
             out[e] = v;
         }
@@ -189,12 +202,14 @@ __global__ void k_tile_sum(EvalArgs a, tile::TileArgs g, int64_t chunks)
         const int4 ck = g.chunk[cell >> 3];
         if (t >= ck.y) continue;
         const int pr = g.parent[ck.x + t], cb = a.child_beg[pr], nc = a.nchild[pr];
+        const double scale = pow(double(1 << ck.z) / a.box->width, double(lane + 1));
         int64_t node = -1;
         for (int k = 0; k < nc; ++k)
             if (static_cast<int>(a.key[cb + k] & 7) == oct) node = cb + k;
         if (node < 0) continue;
-        if (a.want_pot) sum(g.part_a, g.part_d, (node - g.node0) * qd * a.T, int64_t(qd) * a.T, a.LA + node * qd * a.T);
-        if (a.want_field) sum(g.part_b, nullptr, (node - g.node0) * qd * a.T1, int64_t(qd) * a.T1, a.LB + node * qd * a.T1);
+        const int64_t row = (node - g.node0) * qd;
+        if (a.want_pot) sum(g.part_a, g.part_d, row, a.T, scale, a.LA + node * qd * a.T);
+        if (a.want_field) sum(g.part_b, nullptr, row, a.T1, scale, a.LB + node * qd * a.T1);
     }
 }
 

@@ -98,7 +98,7 @@ struct Frags {
 
 // Warps of a full block: as many as the sums' registers (8 per row tile) and
 // the operand buffers in shared memory leave room for.  At 255 registers some
-// of it is still spilled: 80 bytes a thread at p = 10, 190 at 11, 270 at 8, 1,070
+// of it is still spilled: 80 bytes a thread at p = 10, 186 at 11, 234 at 8, 1,058
 // at 12.
 __host__ __device__ constexpr int full_warps(int P) { return P <= 6 ? 16 : P <= 8 ? 12 : P <= 10 ? 8 : 6; }
 
@@ -111,9 +111,9 @@ struct TileArgs {
     const int4* chunk;                    // (first parent, parents, level of the targets, 0)
     int64_t items;                        // chunks x 8 octants (x kParts when split)
     int tpb;                              // targets per tile
-    // split: an item is one part of a tile; its sums go to part_a, part_b and part_d (the order-P sources) [part][row],
-    // row = (node - node0) qdim + component, for k_tile_sum.  Else an item's parts are added to the locals in part
-    // order, the same sums.
+    // split: an item is one part of a tile; its sums go, not yet scaled to the level, to part_a, part_b and part_d (the
+    // order-P sources) [part][row], row = (node - node0) qdim + component, for k_tile_sum.  Else an item's parts are
+    // scaled and added to the locals in part order, the same operations.
     int split;
     int64_t node0, rows;
     cplx *part_a, *part_b, *part_d;

@@ -90,10 +90,6 @@ __device__ __forceinline__ double2 lds2(uint32_t addr)
     return v;
 }
 
-// o + u s with both roundings, so that a part's share is the same number whether
-// it is added here or stored and added by k_tile_sum.
-__device__ __forceinline__ double add_scaled(double o, double u, double s) { return __dadd_rn(o, __dmul_rn(u, s)); }
-
 // The loads that v depends on stay before this point.
 __device__ __forceinline__ void before(double (&v)[4])
 {
@@ -126,15 +122,15 @@ struct Smem {
     static constexpr int ring_m = 16 * CD * 8, ops_d = NW * kRing * ring_m;
     static constexpr int rings = ops_d + kRing * 256 * F::ND;
     static constexpr int lvl = stages > rings ? stages : rings;   // [P + 3] s^n of the level
-    static constexpr int mask = lvl + 8 * up(P + 3, 2) * 2; // [216] x [NW] bytes: a warp's columns with a source
+    static constexpr int fsc = lvl + 8 * up(P + 3, 2) * 2;   // [P + 3] scales of the sums: s^n, or 1 (split: k_tile_sum scales)
+    static constexpr int mask = fsc + 8 * up(P + 3, 2) * 2; // [216] x [NW] bytes: a warp's columns with a source
     static constexpr int used = mask + up(kSlots * NW, 16) * 16;   // [216] slots that occur
     static constexpr int cls = used + 4 * kSlots;           // [216] their rotation classes
     static constexpr int act = cls + up(kSlots, 16) * 16;           // [NW][216]: the warp's slots: index into used | slot << 8
     static constexpr int tgt = act + up(2 * kSlots * NW, 16) * 16; // [8 NW] target node of each tile position
     static constexpr int bars = tgt + 4 * 8 * NW;           // mbarriers: kRing per warp (moments); kOps operators full, empty
     static constexpr int misc = bars + 8 * (kRing * NW + 2 * kOps);   // item, slot count, abort
-    static constexpr int issued = misc + 16;                // last_copy_parity bits: a byte per warp (moments) and operator buffer
-    static constexpr int total = issued + up(NW + kOps, 8) * 8;
+    static constexpr int total = misc + 16;
 };
 
 template<int P, int NW>
@@ -144,7 +140,7 @@ __global__ void __launch_bounds__(32 * NW, 1) k_m2l_tile(EvalArgs a, TileArgs g)
     using S = Smem<P, NW>;
     constexpr int T = F::T, T1 = F::T1, NC = 8 * NW, CS = S::CS, CD = S::CD, NTH = 32 * NW;
     extern __shared__ __align__(128) unsigned char sm[];
-    double* lvl = reinterpret_cast<double*>(sm + S::lvl);
+    double *lvl = reinterpret_cast<double*>(sm + S::lvl), *fsc = reinterpret_cast<double*>(sm + S::fsc);
     unsigned char* mask = sm + S::mask;
     int* used = reinterpret_cast<int*>(sm + S::used);
     unsigned char* cls = sm + S::cls;
@@ -155,7 +151,6 @@ __global__ void __launch_bounds__(32 * NW, 1) k_m2l_tile(EvalArgs a, TileArgs g)
     int* ns_s = reinterpret_cast<int*>(sm + S::misc + 8);
     int* abort_s = reinterpret_cast<int*>(sm + S::misc + 12);
     volatile int* abort = abort_s;
-    unsigned char *issM = sm + S::issued + (threadIdx.x >> 5), *issO = sm + S::issued + NW;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, lr = lane >> 2, lc = lane & 3;
     const int qd = a.qdim, tpb = g.tpb;
@@ -164,7 +159,6 @@ __global__ void __launch_bounds__(32 * NW, 1) k_m2l_tile(EvalArgs a, TileArgs g)
     // moments; operators (R, T, I or the D ring) landed; every warp done with them
     uint64_t *barM = bars + warp * kRing, *barO = bars + NW * kRing, *barE = barO + kOps;
     unsigned char *bufM = sm + warp * S::buf_m, *bufZ = sm + S::z + warp * S::buf_z;
-    if (tid < NW + kOps) sm[S::issued + tid] = 0;
     if (tid == 0) {
         for (int i = 0; i < kRing * NW + kOps; ++i) bar_init(bars + i, 1);
         for (int i = 0; i < kOps; ++i) bar_init(barE + i, NW);
@@ -172,7 +166,10 @@ __global__ void __launch_bounds__(32 * NW, 1) k_m2l_tile(EvalArgs a, TileArgs g)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    uint32_t parM = 0, parO = 0;                            // parities of the next waits, a bit per barrier (barE: as barO)
+    // parities of the next waits, a bit per barrier (barE: as barO); from bit kIssued on, of the copies this thread
+    // issued to each (last_copy_parity)
+    uint32_t parM = 0, parO = 0;
+    constexpr int kIssued = 16;
 
     for (;;) {
         if (tid == 0) *item_s = atomicAdd(g.ctr, 1);
@@ -197,7 +194,10 @@ __global__ void __launch_bounds__(32 * NW, 1) k_m2l_tile(EvalArgs a, TileArgs g)
             }
             tgt[t] = node;
         }
-        if (tid < P + 3) lvl[tid] = pow(double(1 << lt) / a.box->width, double(tid));
+        if (tid < P + 3) {
+            lvl[tid] = pow(double(1 << lt) / a.box->width, double(tid));
+            fsc[tid] = g.split ? 1.0 : lvl[tid];
+        }
         __syncthreads();
         for (int t = warp; t < ck.y; t += NW) {
             const int node = tgt[t];
@@ -256,16 +256,14 @@ __global__ void __launch_bounds__(32 * NW, 1) k_m2l_tile(EvalArgs a, TileArgs g)
         // the moments (coefficients [first, first + count)) of those sources into b
         auto load_moments = [&](int src, unsigned char* b, int first, int count, int stride, int mb) {
             uint64_t* bar = barM + mb;
-            if (lane == 0) {
-                *issM ^= 1u << mb;
-                bar_expect(bar, 8 * count * 16);
-            }
+            if (lane == 0) bar_expect(bar, 8 * count * 16);
+            parM ^= 1u << (kIssued + mb);
             __syncwarp();
             if (lane < 8)
                 bulk(b + lane * stride * 16, src >= 0 ? a.M + (int64_t(src) * qd + bq) * T + first : g.zero, count * 16, bar);
         };
         auto load_ops = [&](int i, int first, int count, int where, int bar) {
-            issO[bar] ^= 1;
+            parO ^= 1u << (kIssued + bar);
             bar_expect(barO + bar, count * 256);
             bulk(sm + where, g.ops + (cls[i] * F::per_class + first) * 32, count * 256, barO + bar);
         };
@@ -302,7 +300,7 @@ __global__ void __launch_bounds__(32 * NW, 1) k_m2l_tile(EvalArgs a, TileArgs g)
 #pragma unroll
             for (int u = 0; u < F::IT; ++u) sum[u][0] = sum[u][1] = sum[u][2] = sum[u][3] = 0.0;
             constexpr int DB = S::DB;
-            // a part's sums, scaled back to the level, to the locals (or the part's own rows)
+            // a part's sums, scaled back to the level, to the locals (or as they are to the part's own rows)
             bool fresh = true;
             auto flush = [&](int part) {
                 const bool set = g.split || fresh;
@@ -334,7 +332,7 @@ __global__ void __launch_bounds__(32 * NW, 1) k_m2l_tile(EvalArgs a, TileArgs g)
                         static_for<0, P + 2>([&](auto jj) {
                             constexpr int j = decltype(jj)::value;
                             if constexpr (j <= P + 1 - pot) {
-                                const double sc = lvl[j + 1];
+                                const double sc = fsc[j + 1];
 #pragma unroll
                                 for (int rt = 0; rt < F::rt(j); ++rt) {
                                     constexpr int u0 = F::inv_tiles(j);
@@ -342,7 +340,7 @@ __global__ void __launch_bounds__(32 * NW, 1) k_m2l_tile(EvalArgs a, TileArgs g)
                                     const int m = 8 * rt + lr;
                                     const double(&u)[4] = sum[u0 + rt];
                                     const cplx o = old[u0 + rt - first];
-                                    if (m <= j) out[j * (j + 1) / 2 + m] = cplx{add_scaled(o.re, u[h], sc), add_scaled(o.im, u[2 + h], sc)};
+                                    if (m <= j) out[j * (j + 1) / 2 + m] = cplx{fma(u[h], sc, o.re), fma(u[2 + h], sc, o.im)};
                                 }
                             }
                         });
@@ -548,9 +546,8 @@ __global__ void __launch_bounds__(32 * NW, 1) k_m2l_tile(EvalArgs a, TileArgs g)
                     for (int t = 0; t < F::DT; ++t) old[t] = !g.split && 8 * t + lr < T ? out[8 * t + lr] : cplx{0, 0};
 #pragma unroll
                     for (int t = 0; t < F::DT; ++t) {
-                        const double sc = lvl[order[t] + 1];
-                        if (8 * t + lr < T)
-                            out[8 * t + lr] = cplx{add_scaled(old[t].re, sum[t][h], sc), add_scaled(old[t].im, sum[t][2 + h], sc)};
+                        const double sc = fsc[order[t] + 1];
+                        if (8 * t + lr < T) out[8 * t + lr] = cplx{fma(sum[t][h], sc, old[t].re), fma(sum[t][2 + h], sc, old[t].im)};
                     }
                 }
 #pragma unroll
@@ -641,14 +638,17 @@ __global__ void __launch_bounds__(32 * NW, 1) k_m2l_tile(EvalArgs a, TileArgs g)
         }
         __syncthreads();
         if (*abort) {
-            // copies in flight land before shared memory is released
-            if (lane == 0) drain_copies(*issM, kRing, kDrainPolls, [&](int b, uint32_t parity) { return bar_try(barM + b, parity); });
+            // copies in flight land before shared memory is released; an operator buffer's copies come from several warps
+            if (lane == 0) drain_copies(parM >> kIssued, kRing, kDrainPolls, [&](int b, uint32_t parity) { return bar_try(barM + b, parity); });
             if (tid == 0) {
                 atomicExch(a.wait_err, 1);
-                uint32_t issued = 0;
-                for (int b = 0; b < kOps; ++b) issued |= uint32_t(issO[b]) << b;
-                drain_copies(issued, kOps, kDrainPolls, [&](int b, uint32_t parity) { return bar_try(barO + b, parity); });
+                *ns_s = 0;
             }
+            __syncthreads();
+            if (lane == 0) atomicXor(ns_s, static_cast<int>(parO >> kIssued));
+            __syncthreads();
+            if (tid == 0)
+                drain_copies(static_cast<uint32_t>(*ns_s), kOps, kDrainPolls, [&](int b, uint32_t parity) { return bar_try(barO + b, parity); });
             break;
         }
     }
