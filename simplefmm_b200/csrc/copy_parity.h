@@ -19,6 +19,16 @@ namespace sfmm {
 // has landed; else when it lands.  The other parity never completes.
 SFMM_CP_HD uint32_t last_copy_parity(uint32_t issued, int b) { return (issued >> b & 1u) ^ 1u; }
 
+// The bits of a warp that gives up, from those of its waits: of a pass's copies,
+// in turn on `ring` barriers, the first `waited` were waited for (or counted as
+// such) and `issued` issued; the rest flip their barrier's bit.
+SFMM_CP_HD uint32_t in_flight(int waited, int issued, int ring)
+{
+    uint32_t bits = 0;
+    for (int s = waited; s < issued; ++s) bits ^= 1u << (s % ring);
+    return bits;
+}
+
 // Waits for barriers 0 .. n - 1 with at most `polls` polls each; try_wait(b,
 // parity) is one poll.  False when a barrier's polls ran out.
 template<typename TryWait>

@@ -98,7 +98,7 @@ struct Frags {
 
 // Warps of a full block: as many as the sums' registers (8 per row tile) and
 // the operand buffers in shared memory leave room for.  At 255 registers some
-// of it is still spilled: 80 bytes a thread at p = 10, 186 at 11, 234 at 8, 1,058
+// of it is still spilled: 76 bytes a thread at p = 10, 186 at 11, 266 at 8, 1,082
 // at 12.
 __host__ __device__ constexpr int full_warps(int P) { return P <= 6 ? 16 : P <= 8 ? 12 : P <= 10 ? 8 : 6; }
 

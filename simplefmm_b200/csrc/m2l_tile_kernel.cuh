@@ -166,8 +166,8 @@ __global__ void __launch_bounds__(32 * NW, 1) k_m2l_tile(EvalArgs a, TileArgs g)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    // parities of the next waits, a bit per barrier (barE: as barO); from bit kIssued on, of the copies this thread
-    // issued to each (last_copy_parity)
+    // parities of the next waits, a bit per barrier (barE: as barO); in parO, from bit kIssued on, of the operator copies
+    // this thread issued to each (last_copy_parity; a warp's moments follow from its place in the pass, in_flight)
     uint32_t parM = 0, parO = 0;
     constexpr int kIssued = 16;
 
@@ -257,7 +257,6 @@ __global__ void __launch_bounds__(32 * NW, 1) k_m2l_tile(EvalArgs a, TileArgs g)
         auto load_moments = [&](int src, unsigned char* b, int first, int count, int stride, int mb) {
             uint64_t* bar = barM + mb;
             if (lane == 0) bar_expect(bar, 8 * count * 16);
-            parM ^= 1u << (kIssued + mb);
             __syncwarp();
             if (lane < 8)
                 bulk(b + lane * stride * 16, src >= 0 ? a.M + (int64_t(src) * qd + bq) * T + first : g.zero, count * 16, bar);
@@ -391,6 +390,7 @@ __global__ void __launch_bounds__(32 * NW, 1) k_m2l_tile(EvalArgs a, TileArgs g)
             };
             if (na > 0) load_e();
             uint32_t parE = parO;                           // parities of the operators' earlier uses (T, I)
+            bool counted = false;                           // given up with the k-th slot's moments counted as waited for
             for (int i = 0; i < ns; ++i) {
                 const bool on = (cur & 255) == i;            // the warp has a source in this slot
                 const int here = (cur >> 8) / kPartSlots;    // its part
@@ -405,7 +405,10 @@ __global__ void __launch_bounds__(32 * NW, 1) k_m2l_tile(EvalArgs a, TileArgs g)
                     parM ^= 1u;
                 }
                 ok = ok && bar_wait(barO, parO & 1u, abort);
-                if (!ok) break;
+                if (!ok) {
+                    counted = on;
+                    break;
+                }
                 if (on) {
                     const uint32_t M = after(m32), ops = after(ops32), lv = s32(lvl);
                     static_for<0, P>([&](auto nn) {
@@ -520,7 +523,10 @@ __global__ void __launch_bounds__(32 * NW, 1) k_m2l_tile(EvalArgs a, TileArgs g)
                 if (on && (k == na || (cur >> 8) / kPartSlots != here)) flush(here);   // the part's last slot
                 parO ^= 1u | 1u << tb | 1u << ib;
             }
-            if (!ok) *abort = 1;
+            if (!ok) {
+                parM ^= in_flight(k + counted, imin(k + 1, na), 1);
+                *abort = 1;
+            }
             if (fresh) flush(part0);                        // no source at all: zeros
         }
         __syncthreads();
@@ -565,6 +571,7 @@ __global__ void __launch_bounds__(32 * NW, 1) k_m2l_tile(EvalArgs a, TileArgs g)
             double2 e[F::DK];                               // s^P e^{i m phi} of the azimuth, m = 4 kc + lc
             uint32_t parE = parO;                           // parities of the operators' earlier uses
             int k = 0, az = -1;
+            bool counted = false;                           // as in the first pass
             auto load_e = [&](int s) {
                 const double2* eil = phases(s);
 #pragma unroll
@@ -584,7 +591,10 @@ __global__ void __launch_bounds__(32 * NW, 1) k_m2l_tile(EvalArgs a, TileArgs g)
                     parM ^= 1u << mb;
                 }
                 ok = ok && bar_wait(barO + b, parO >> b & 1u, abort);
-                if (!ok) break;
+                if (!ok) {
+                    counted = on;
+                    break;
+                }
                 if (on) {
                     const uint32_t M = after(ring32 + mb * S::ring_m), ops = after(s32(sm + S::ops_d) + lane * 8 + b * 256 * F::ND);
                     double xr[F::DK], xi[F::DK];
@@ -633,13 +643,16 @@ __global__ void __launch_bounds__(32 * NW, 1) k_m2l_tile(EvalArgs a, TileArgs g)
                     parE ^= 1u << pb;
                 }
             }
-            if (!ok) *abort = 1;
+            if (!ok) {
+                parM ^= in_flight(k + counted, imin(k + kRing, na), kRing);
+                *abort = 1;
+            }
             if (g.split && na == 0) flush(part0);
         }
         __syncthreads();
         if (*abort) {
             // copies in flight land before shared memory is released; an operator buffer's copies come from several warps
-            if (lane == 0) drain_copies(parM >> kIssued, kRing, kDrainPolls, [&](int b, uint32_t parity) { return bar_try(barM + b, parity); });
+            if (lane == 0) drain_copies(parM, kRing, kDrainPolls, [&](int b, uint32_t parity) { return bar_try(barM + b, parity); });
             if (tid == 0) {
                 atomicExch(a.wait_err, 1);
                 *ns_s = 0;

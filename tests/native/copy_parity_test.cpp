@@ -55,6 +55,23 @@ int main()
         flying += out > 0;
     }
     if (checked < 15000 || flying < 5000) return 5;
+    // passes of na copies in turn on `ring` barriers, `ring` ahead, given up before or after the wait for copy k: the
+    // waits' bits and in_flight give the issues' bits
+    for (int ring : {1, 2, 4})
+        for (int na = 0; na < 12; ++na)
+            for (int stop = 0; stop <= na; ++stop)
+                for (int counted = 0; counted <= (stop < na); ++counted) {
+                    unsigned waits = rng() & ((1u << ring) - 1), issues = waits;   // bits left by earlier passes: all landed
+                    auto issue = [&](int s) { issues ^= 1u << (s % ring); };
+                    for (int s = 0; s < ring && s < na; ++s) issue(s);
+                    for (int k = 0; k < stop; ++k) {
+                        waits ^= 1u << (k % ring);
+                        if (k + ring < na) issue(k + ring);
+                    }
+                    if (counted) waits ^= 1u << (stop % ring);
+                    const int issued = stop + ring < na ? stop + ring : na;
+                    if ((waits ^ sfmm::in_flight(stop + counted, issued, ring)) != issues) return 6;
+                }
     std::printf("copy parity ok\n");
     return 0;
 }

@@ -1,5 +1,6 @@
 """CPU test of the phases a giving-up kernel waits for (csrc/copy_parity.h):
-barriers whose copies have landed cost one poll, the others are waited for."""
+barriers whose copies have landed cost one poll, the others are waited for, and
+the waits' parities at any point of a pass give the issues'."""
 import subprocess
 from pathlib import Path
 
