@@ -177,9 +177,9 @@ struct fmm_server {
 
 // Bytes of part sums for requests just admitted together (mu held): what they
 // can use, if that fits beside the running requests and the queued ones that
-// the idle workers could take; else none.  A request is never refused or kept
-// waiting for part sums: without them its M2L runs a tile's parts in turn, to
-// the same results.
+// the idle workers could take; else none.  So no request is refused for part
+// sums, and none that is queued now waits for them: without them an M2L runs a
+// tile's parts in turn, to the same results.
 size_t fmm_server::grant_parts(const std::vector<std::shared_ptr<Request>>& rs) const
 {
     size_t want = 0;
